@@ -28,16 +28,14 @@ NVCCFLAGS = ARCH + ["-std=c++20", "-O3", "-lineinfo", "-Xcompiler", "-fPIC",
                     "-Xcompiler", "-ffp-contract=off", "--expt-relaxed-constexpr"]
 
 HOST_SOURCES = ["planner.cpp", "stream_plan.cpp", "executor.cpp", "sweep.cpp", "server.cpp",
-                "host_blocks.cpp", "capi.cpp"]
-TSTREAM2_SOURCES = [f"tstream2_hb{hb}_k{k}.cu" for hb in (1, 3, 5, 7) for k in (0, 8)]
+                "host_blocks.cpp", "tensor_map.cpp", "capi.cpp"]
+TRING_SOURCES = [f"tring_hb{hb}_w{w}.cu" for hb, ws in ((1, (4, 8, 16)), (3, (8, 12, 16)), (5, (8, 12, 16)),
+                                                      (7, (12, 16))) for w in ws]
 TSOLVE_SOURCES = ([f"tsolve_hb{hb}.cu" for hb in (1, 3, 5, 7, 9, 11)]
                   + [f"tsolve64_hb{hb}.cu" for hb in (1, 3, 5, 7, 9, 11)])
-CUDA_SOURCES = TSTREAM2_SOURCES + TSOLVE_SOURCES + ["kernels.cu", "stream.cu", "stream_hb1.cu", "stream_hb3.cu", "stream_hb5.cu",
-                "stream_hb7.cu", "tstream_hb1.cu", "tstream_hb3.cu",
-                "tstream_hb5.cu", "tstream_hb7.cu", "tstream_hb1_g.cu", "tstream_hb3_g.cu",
-                "tstream_hb5_g.cu", "tstream_hb7_g.cu", "tscore_hb1.cu", "tscore_hb3.cu",
-                "tscore_hb5.cu", "tscore_hb7.cu", "noalloc.cu", "score.cu",
-                "peak.cu", "gpu_planner.cu", "refine64.cu"]
+CUDA_SOURCES = TRING_SOURCES + TSOLVE_SOURCES + ["kernels.cu", "stream.cu", "stream_hb1.cu", "stream_hb3.cu",
+                "stream_hb5.cu", "stream_hb7.cu", "tscore_hb1.cu", "tscore_hb3.cu", "tscore_hb5.cu",
+                "tscore_hb7.cu", "noalloc.cu", "score.cu", "peak.cu", "gpu_planner.cu", "refine64.cu"]
 
 
 def cuda_home() -> str:

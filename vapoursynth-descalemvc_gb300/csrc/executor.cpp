@@ -15,6 +15,7 @@
 #include "score.cuh"
 #include "stream.cuh"
 #include "stream_plan.hpp"
+#include "tensor_map.hpp"
 
 #include <cuda_runtime.h>
 
@@ -104,16 +105,18 @@ struct DevicePlan {
     std::vector<int> chunk_first_block64;
     dev::StreamPlanView stream_view64{};
     dev::StreamPlanView stream_view{};
-    // Grouped forward records of the chunk-delayed transposing kernels
+    // Grouped forward records of the fused scoring kernels
     // (StreamPack::forward_groups), when the plan has them: their union.
     int stream_union = 0;
     dev::StreamPlanView stream_view_g{};
-    bool stream_p = false;          // paired transposing 2D kernels admitted
-    dev::StreamPlanView stream_view2{};
+    // Chunk-delayed 2D kernels with the ring in tensor memory
+    // (StreamPack::ring_forward), when the plan admits them: their window.
+    int ring_window = 0;
+    dev::StreamPlanView ring_view{};
     // Chunk-delayed transposing passes may split vectors into segments
     // (stream_plan.hpp); the ring's first block of each chunk.
     bool stream_seg = false;
-    std::vector<int> chunk_first_block;
+    std::vector<int> chunk_first_block, ring_first_block;
     // Two-pass transposing kernels in segments (StreamPack::exact_margin).
     int exact_margin = 0;
     std::size_t bytes = 0;
@@ -126,7 +129,7 @@ struct PlanImage {
     std::vector<std::size_t> offsets;
     StreamPack pack;
     StreamPack64 pack64;
-    std::size_t at_records = 0, at_paired = 0, at_records64 = 0, at_groups = 0;
+    std::size_t at_records = 0, at_ring = 0, at_records64 = 0, at_groups = 0;
 };
 
 PlanImage plan_image(const AxisPlan &p) {
@@ -149,7 +152,7 @@ PlanImage plan_image(const AxisPlan &p) {
     img.pack64 = pack_stream_plan64(p, kStreamChunk, kStreamRing, tsolve_supports(p.half_bandwidth));
     const StreamPack &pack = img.pack;
     const StreamPack64 &pack64 = img.pack64;
-    std::size_t &at_records = img.at_records, &at_paired = img.at_paired, &at_records64 = img.at_records64,
+    std::size_t &at_records = img.at_records, &at_ring = img.at_ring, &at_records64 = img.at_records64,
                 &at_groups = img.at_groups;
     if (pack.eligible || pack.exact) {
         at_records = parts.size();
@@ -160,10 +163,10 @@ PlanImage plan_image(const AxisPlan &p) {
             parts.push_back({pack.forward_groups.data(), pack.forward_groups.size() * 4});
             parts.push_back({pack.backward_groups.data(), pack.backward_groups.size() * 4});
         }
-        if (pack.paired) {
-            at_paired = parts.size();
-            parts.push_back({pack.paired_forward.data(), pack.paired_forward.size() * 4});
-            parts.push_back({pack.paired_backward.data(), pack.paired_backward.size() * 4});
+        if (pack.ring_window) {
+            at_ring = parts.size();
+            parts.push_back({pack.ring_forward.data(), pack.ring_forward.size() * 4});
+            parts.push_back({pack.ring_backward.data(), pack.ring_backward.size() * 4});
         }
     }
     if (pack64.eligible) {
@@ -188,7 +191,7 @@ void finish_plan(DevicePlan *dp, const AxisPlan &p, const PlanImage &img, char *
     const StreamPack &pack = img.pack;
     const StreamPack64 &pack64 = img.pack64;
     const std::vector<std::size_t> &offsets = img.offsets;
-    const std::size_t at_records = img.at_records, at_paired = img.at_paired, at_records64 = img.at_records64,
+    const std::size_t at_records = img.at_records, at_ring = img.at_ring, at_records64 = img.at_records64,
                       at_groups = img.at_groups;
     const std::size_t total = img.bytes.size();
     auto &v = dp->view;
@@ -233,14 +236,16 @@ void finish_plan(DevicePlan *dp, const AxisPlan &p, const PlanImage &img, char *
             dp->stream_view_g.backward_stride = (4 * p.half_bandwidth + 3) / 4;
             dp->stream_view_g.backward = reinterpret_cast<const float *>(base + offsets[at_groups + 1]);
         }
-        if (pack.paired) {
-            dp->stream_p = true;
-            auto &pv = dp->stream_view2;
-            pv = sv;
-            pv.forward_stride = pack.paired_forward_stride;
-            pv.backward_stride = pack.paired_backward_stride;
-            pv.forward = reinterpret_cast<const float *>(base + offsets[at_paired]);
-            pv.backward = reinterpret_cast<const float *>(base + offsets[at_paired + 1]);
+        if (pack.ring_window) {
+            dp->ring_window = pack.ring_window;
+            dp->ring_first_block = pack.ring_first_block;
+            auto &rv = dp->ring_view;
+            rv = sv;
+            rv.window = pack.ring_window;
+            rv.forward_stride = 2 + pack.ring_window + p.half_bandwidth;
+            rv.backward_stride = p.half_bandwidth;
+            rv.forward = reinterpret_cast<const float *>(base + offsets[at_ring]);
+            rv.backward = reinterpret_cast<const float *>(base + offsets[at_ring + 1]);
         }
     }
     if (pack64.eligible) {
@@ -549,9 +554,8 @@ struct Executor::Impl {
     // DSMVC_GB_STREAM=0 keeps every plan on the sequential kernels (the
     // counterpart of the reference's DSMVC_GPU_SOLVE_PARTITION switch).
     bool allow_stream = true;
-    // DSMVC_GB_PAIRED=1 runs admitted 2D planes on the paired transposing
-    // kernels (64 vectors per warp); the unpaired ones (32 per warp) are the
-    // default, faster on GB300 at the occupancy the paired ones reach.
+    // DSMVC_GB_PAIRED=1 runs every chunk-delayed 2D pass with two vectors a
+    // lane, in whole vectors (kind 4).
     bool allow_paired = false;
     // DSMVC_GB_EXACT=1 runs every admitted 2D pass on the two-pass
     // transposing kernels; otherwise they serve the plans the chunk-delayed
@@ -671,6 +675,7 @@ struct Executor::Impl {
         std::uint64_t bytes;
         int record_floats;
         int threads;
+        int per_lane;
     };
     // CTA size per launch group, keyed by (pass, kind, hb, in, out, variant);
     // groups not listed take the default size of their kernel.
@@ -727,15 +732,28 @@ bool stream_row_ok(const DevicePlan &dp, dev::Sample in) {
     return in == dev::Sample::f32;
 }
 
-// Launch-group variant of a transposing pass.  Chunk-delayed kernels: the
-// union of grouped records (12, 16), else 8 for the window-8 kernels
-// (compile-time gather), else 0.  Paired and two-pass kernels: 1 runs the
-// window-8 kernels (for the two-pass ones also the grouped refill).
+// Variant bit of the chunk-delayed kinds: the pass writes the tiled
+// intermediate.
+constexpr int kTiled = 32;
+
+// Launch-group variant of a transposing pass.  Chunk-delayed kernels (3, 4):
+// their window.  Two-pass kernels: 1 runs the window-8 kernels with the
+// grouped refill.
 int compiled_window(const DevicePlan &dp, int kind) {
     if (kind == 5) return dp.stream_xg ? 1 : 0;
-    if (kind == 3 && dp.stream_union) return dp.stream_union;
-    return dp.stream_view.window == 8 ? (kind == 3 ? 8 : 1) : 0;
+    return dp.ring_window;
 }
+
+// Launches of at least this many warps an SM (at one vector a lane) run two
+// vectors a lane: a record's load then serves both, and four warps an SM stay.
+// Measured on one GB300: 64 YUV420P16 1080p frames (14 warps an SM) 546 us a
+// batch at one vector a lane, 536 at two; 32 4K Float32 frames (14) 640 and
+// 604; 24 YUV420P8 720x480 frames (4) 95.6 and 132.
+constexpr int kPairingWarps = 8;
+
+// The chunk-delayed transposing kinds: 3, whose vectors a lane compile()
+// chooses, and 4, two.
+bool ring_kind(int kind) { return kind == 3 || kind == 4; }
 
 std::string kernel_name(const GroupKey &k);
 
@@ -745,8 +763,9 @@ int Executor::Impl::fused_window(const DevicePlan &dp) const {
     if (!allow_stream || prefer_exact || !dp.stream || !dp.stream_t) return -1;
     const int hb = dp.stream_view.half_bandwidth;
     if (hb < 1 || hb > 7) return -1;
-    const int w = compiled_window(dp, 3);
-    return w == 0 || w == 8 || w == 12 || w == 16 ? w : -1;
+    // The union of grouped records, else 8 (compile-time gather), else 0.
+    if (dp.stream_union) return dp.stream_union;
+    return dp.stream_view.window == 8 ? 8 : 0;
 }
 
 namespace {
@@ -837,7 +856,7 @@ std::vector<Item> segment_items(const std::vector<Item> &items, int vectors_per_
                 if (s > 1) {
                     it.stream.chunk_begin = begin;
                     it.stream.chunk_end = end;
-                    it.stream.first_sample = begin > 0 ? dp->chunk_first_block[static_cast<std::size_t>(begin - 1)] : 0;
+                    it.stream.first_sample = begin > 0 ? dp->ring_first_block[static_cast<std::size_t>(begin - 1)] : 0;
                 }
                 out.push_back(it);
             }
@@ -852,7 +871,7 @@ std::vector<Item> segment_items(const std::vector<Item> &items, int vectors_per_
 void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                              const std::function<char *(std::size_t)> &scratch, std::uint32_t *status,
                              const Tuning *tuning, int vectors_per_warp) {
-    const bool paired = vectors_per_warp ? vectors_per_warp == 64 : allow_paired;
+    if (!vectors_per_warp && allow_paired) vectors_per_warp = 64;
     auto &temporaries = out.temporaries;
     // Per task: which kernels run each pass, and the scratch they need.
     struct Route {
@@ -863,7 +882,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
         // adjacent vectors.
         // 2D passes: 0 sequential, 3 chunk-delayed, 4 paired chunk-delayed,
         // 5 two-pass transposing.
-        bool transposed = false;
+        bool transposed = false, tiled = false;
         // Float64 planes whose plans both admit the Float64 two-pass
         // transposing kernels (kind 6): a transposed Float64 intermediate.
         bool transposed64 = false;
@@ -915,9 +934,9 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
             r.transposed = true;
             auto pass_kind = [&](const DevicePlan &dp) {
                 if (!allow_stream) return 0;
-                const bool delayed = dp.stream && dp.stream_t;
+                const bool delayed = dp.stream && dp.ring_window;
                 if (dp.stream_x && (prefer_exact || !delayed)) return 5;
-                if (delayed) return paired && dp.stream_p ? 4 : 3;
+                if (delayed) return vectors_per_warp == 64 ? 4 : 3;
                 return 0;
             };
             r.h_kind = pass_kind(*r.h);
@@ -928,7 +947,11 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                     throw std::invalid_argument("fused scoring needs a chunk-delayed Float32 columns pass");
                 r.v_kind = 9;
             }
-            r.mid_stride = (static_cast<std::size_t>(v->source_size) + 3) / 4 * 4;
+            // Between two chunk-delayed passes the intermediate is tiled,
+            // [row / 32][destination][row mod 32].
+            r.tiled = ring_kind(r.h_kind) && ring_kind(r.v_kind) && v->source_size >= 32;
+            const std::size_t whole = r.tiled ? 32 : 4;
+            r.mid_stride = (static_cast<std::size_t>(v->source_size) + whole - 1) / whole * whole;
             r.mid = bytes;
             bytes += align_up(r.mid_stride * static_cast<std::size_t>(h->destination_size) * 4);
             // Forward values of the second pass when the output cannot hold
@@ -1029,6 +1052,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
         std::uint64_t bytes = 0;
         const DevicePlan *plan = nullptr;   // chunk-delayed transposing passes
         int tiles = 0;                      // fused scoring: CTAs of the job
+        int tile_vectors = 0;               // tiled intermediates: their vectors
     };
     std::map<GroupKey, std::vector<Item>> groups;
     for (std::size_t t = 0; t < tasks.size(); ++t) {
@@ -1113,8 +1137,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                 * sample_bytes(task.sample);
             if (r.h_kind) {
                 auto &j = hi.stream;
-                j.plan = r.h_kind == 4 ? r.h->stream_view2
-                       : r.h_kind == 3 && r.h->stream_union ? r.h->stream_view_g : r.h->stream_view;
+                j.plan = r.h_kind == 5 ? r.h->stream_view : r.h->ring_view;
                 j.in = task.input; j.in_elem = 1; j.in_vec = task.input_stride;
                 j.out = mid; j.out_elem = pitch; j.out_vec = 1;
                 j.y = mid; j.y_elem = pitch;                // forward values in place
@@ -1122,7 +1145,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                 j.conv = conv;
                 hi.plan = r.h;
                 auto &group = groups[{0, r.h_kind, h->half_bandwidth, task.sample, dev::Sample::f32,
-                                      compiled_window(*r.h, r.h_kind)}];
+                                      compiled_window(*r.h, r.h_kind) | (r.tiled ? kTiled : 0)}];
                 if (r.h_kind == 5)
                     push_segments(group, hi, r.h->chunk_first_block, r.h->exact_margin, h->destination_size, r.seg_h,
                                   base + r.yseg_h, pitch, 4);
@@ -1151,9 +1174,9 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                 groups[{1, 9, v->half_bandwidth, dev::Sample::f32, dev::Sample::f32, fused_window(*r.v)}].push_back(vi);
             } else if (r.v_kind) {
                 auto &j = vi.stream;
-                j.plan = r.v_kind == 4 ? r.v->stream_view2
-                       : r.v_kind == 3 && r.v->stream_union ? r.v->stream_view_g : r.v->stream_view;
-                j.in = mid; j.in_elem = 1; j.in_vec = pitch;
+                j.plan = r.v_kind == 5 ? r.v->stream_view : r.v->ring_view;
+                j.in = mid; j.in_elem = 1; j.in_vec = r.tiled ? 32 : pitch;
+                vi.tile_vectors = r.tiled ? h->destination_size : 0;
                 j.out = task.output; j.out_elem = task.output_stride; j.out_vec = 1;
                 if (r.fwd_stride) {
                     j.y = reinterpret_cast<float *>(base + r.fwd);
@@ -1268,9 +1291,10 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
     for (auto &[key, items] : groups) {
         const bool fused = key.kind == 9;
         const bool is_stream = (key.kind >= 2 && key.kind <= 6) || fused;
+        const bool ring = ring_kind(key.kind);
         int per_block = key.kind == 2 ? stream_block : fused ? kScoreCtaThreads
-                      : is_stream ? tstream_threads : kSeqThreads;
-        if (tuning && key.kind != 2 && key.kind <= 6) {
+                      : ring ? kTRingThreads : is_stream ? tstream_threads : kSeqThreads;
+        if (tuning && key.kind != 2 && !ring && key.kind <= 6) {
             const GroupTuple g{key.pass, key.kind, key.hb, static_cast<int>(key.in), static_cast<int>(key.out),
                                key.variant};
             if (auto it = tuning->find(g); it != tuning->end()) per_block = it->second;
@@ -1285,7 +1309,6 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
         // copies), so only plan changes round up to a whole CTA.
         const bool by_warp = (key.kind >= 3 && key.kind <= 6) || fused;
         const int warps_per_cta = per_block / 32;
-        const int vectors_per_warp = key.kind == 4 ? 64 : 32;
         // Jobs of one plan stay together (they share record copies); plans
         // with the longest vectors come first, so that the CTAs that take
         // longest start in the first wave and the launch's tail is short
@@ -1296,7 +1319,21 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                 if (na != nb) return na > nb;
                 return a.stream.plan.forward < b.stream.plan.forward;
             });
-        if (key.kind == 3) items = segment_items(items, vectors_per_warp, segment_mode, warp_slots);
+        int per_lane = 1;
+        if (key.kind == 4) {
+            per_lane = 2;
+        } else if (key.kind == 3) {
+            // The split does not depend on the vectors a lane: neither do the
+            // results.
+            items = segment_items(items, 32, segment_mode, warp_slots);
+            long warps = 0;
+            for (const auto &it : items) warps += (it.stream.vectors + 31) / 32;
+            if (!vectors_per_warp && warps >= kPairingWarps * static_cast<long>(warp_slots / kTResidentWarps))
+                per_lane = 2;
+        }
+        if (ring)
+            for (auto &it : items)
+                map_input(it.stream, key.in, it.stream.plan.source_size, it.tile_vectors, per_lane);
         int warps = 0;
         const float *run_plan = nullptr;
         int run_chunk = 0;
@@ -1315,7 +1352,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                 run_plan = it.stream.plan.forward;
                 run_chunk = it.stream.chunk_begin;
                 it.stream.first_block = warps;     // first warp of the job
-                warps += (vectors + vectors_per_warp - 1) / vectors_per_warp;
+                warps += (vectors + 32 * per_lane - 1) / (32 * per_lane);
                 blocks = (warps + warps_per_cta - 1) / warps_per_cta;
             } else {
                 if (is_stream) it.stream.first_block = blocks; else it.axis.first_block = blocks;
@@ -1335,7 +1372,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
         }
         if (count)
             launches.push_back({key.pass, key.kind, key.hb, key.in, key.out, key.variant, offset, count, blocks,
-                                bytes_moved, record_floats, per_block});
+                                bytes_moved, record_floats, per_block, per_lane});
     }
     out.tasks = tasks.size();
 }
@@ -1373,13 +1410,9 @@ void Executor::Impl::launch(const Compiled &c, const char *device_table, cudaStr
         } else if (l.kind == 5) {
             rc = launch_tsolve(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.threads,
                                l.hb, l.variant ? 8 : 0, l.in, l.out, l.record_floats, stream);
-        } else if (l.kind == 4) {
-            rc = launch_tstream2(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks,
-                                 l.threads, l.hb, l.variant ? 8 : 0, l.in, l.out, l.record_floats, stream);
-        } else if (l.kind == 3) {
-            rc = launch_tstream(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks,
-                                l.threads, l.hb, l.variant, l.in, l.out, l.record_floats,
-                                stream);
+        } else if (ring_kind(l.kind)) {
+            rc = launch_tring(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
+                              l.variant & 31, l.per_lane, (l.variant & kTiled) != 0, l.in, l.out, stream);
         } else if (l.kind == 2) {
             rc = launch_stream(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks,
                                l.hb, kStreamChunk, l.pass == 0, l.in, l.out, l.record_floats,

@@ -33,39 +33,6 @@ int launch_stream(const dev::StreamJob *jobs, int job_count, int total_blocks, i
 
 namespace dsmvc_gb {
 
-int launch_tstream_hb1(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream_hb3(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream_hb5(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream_hb7(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-
-int launch_tstream2_hb1_k0(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream2_hb1_k8(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream2_hb3_k0(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream2_hb3_k8(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream2_hb5_k0(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream2_hb5_k8(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream2_hb7_k0(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream2_hb7_k8(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
-
-int launch_tstream2(const dev::StreamJob *jobs, int job_count, int total_blocks, int threads, int half_bandwidth,
-                    int window, dev::Sample in, dev::Sample out, int record_floats, void *stream) {
-    const bool k8 = window == 8;
-#define DSMVC_PAIRED(H)                                                                                        \
-    case H:                                                                                                    \
-        return k8 ? launch_tstream2_hb##H##_k8(jobs, job_count, total_blocks, threads, in, out, record_floats, \
-                                               stream)                                                         \
-                  : launch_tstream2_hb##H##_k0(jobs, job_count, total_blocks, threads, in, out, record_floats, \
-                                               stream);
-    switch (half_bandwidth) {
-        DSMVC_PAIRED(1)
-        DSMVC_PAIRED(3)
-        DSMVC_PAIRED(5)
-        DSMVC_PAIRED(7)
-    default: return static_cast<int>(cudaErrorInvalidValue);
-    }
-#undef DSMVC_PAIRED
-}
-
 int launch_tsolve_hb1(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
 int launch_tsolve_hb3(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
 int launch_tsolve_hb5(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
@@ -111,29 +78,43 @@ int launch_tsolve(const dev::StreamJob *jobs, int job_count, int total_blocks, i
     }
 }
 
-int launch_tstream_g_hb1(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream_g_hb3(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream_g_hb5(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tstream_g_hb7(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
+int launch_tring_hb1_w4(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_tring_hb1_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_tring_hb1_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_tring_hb3_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_tring_hb3_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_tring_hb3_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_tring_hb5_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_tring_hb5_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_tring_hb5_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_tring_hb7_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_tring_hb7_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
 
-int launch_tstream(const dev::StreamJob *jobs, int job_count, int total_blocks, int threads, int half_bandwidth,
-                   int window, dev::Sample in, dev::Sample out, int record_floats, void *stream) {
-    if (window > 8) {
-        switch (half_bandwidth) {
-        case 1: return launch_tstream_g_hb1(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-        case 3: return launch_tstream_g_hb3(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-        case 5: return launch_tstream_g_hb5(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-        case 7: return launch_tstream_g_hb7(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-        default: return static_cast<int>(cudaErrorInvalidValue);
-        }
-    }
-    switch (half_bandwidth) {
-    case 1: return launch_tstream_hb1(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-    case 3: return launch_tstream_hb3(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-    case 5: return launch_tstream_hb5(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-    case 7: return launch_tstream_hb7(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-    default: return static_cast<int>(cudaErrorInvalidValue);
-    }
+int launch_tring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
+                 int per_lane, bool tiled, dev::Sample in, dev::Sample out, void *stream) {
+    if (half_bandwidth == 1 && window == 4)
+        return launch_tring_hb1_w4(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 1 && window == 8)
+        return launch_tring_hb1_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 1 && window == 16)
+        return launch_tring_hb1_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 3 && window == 8)
+        return launch_tring_hb3_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 3 && window == 12)
+        return launch_tring_hb3_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 3 && window == 16)
+        return launch_tring_hb3_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 5 && window == 8)
+        return launch_tring_hb5_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 5 && window == 12)
+        return launch_tring_hb5_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 5 && window == 16)
+        return launch_tring_hb5_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 7 && window == 12)
+        return launch_tring_hb7_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 7 && window == 16)
+        return launch_tring_hb7_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    return static_cast<int>(cudaErrorInvalidValue);
 }
 
 int launch_tscore_hb1(const dev::StreamJob *, int, int, int, int, void *);

@@ -30,6 +30,11 @@ struct StreamPlanView {
 };
 
 struct StreamJob {
+    // Kernels with the ring in tensor memory: the tensor map of the input, used
+    // when `mapped`: 1 a plane of contiguous vectors, 2 the intermediate in
+    // tiles of 32 samples.
+    alignas(64) unsigned char map[128];
+    std::int32_t mapped;
     StreamPlanView plan;
     const void *in;
     std::int64_t in_elem, in_vec;
@@ -79,36 +84,30 @@ int stream_threads();
 bool stream_supports(int half_bandwidth);
 constexpr int kStreamChunk = 32;     // destinations per register chunk
 constexpr int kStreamRing = 32;      // source samples held per thread
-// Ring row pitches (floats) of the transposing kernels, unpaired and paired;
-// the host stores each destination's window offset in the ring, (s0 mod 32)
-// times the pitch (in floats, resp. float2 for the paired kernels), in its
-// forward record.
+// Source samples held per vector by the kernels with the ring in tensor
+// memory (a multiple of 16; the first 16 stored again and two chunks of
+// forward values fill 128 columns).
+constexpr int kRingColumns = 48;
+// Ring row pitch (floats) of the transposing kernels with the ring in shared
+// memory; the host stores each destination's window offset in the ring,
+// (s0 mod 32) times the pitch, in its forward record.
 constexpr int kTRingPitch = 34;
-constexpr int kPairedRingPitch = 66;
 // `chunk` is 32 or 64; contiguous = the vector's samples are adjacent
 // (rows: f32/u8/u16 in, f32 out); otherwise columns (f32 in; f32/u8/u16 out).
-// Transposing 2D passes (tstream_impl.cuh): vectors with adjacent samples
-// in, destination-major output with the vectors adjacent.  Every job of one
-// launch has the same window when window == 8 (unrolled gather); window 12
-// or 16: every job's plan view carries grouped records with that union
-// (StreamPack::forward_groups).  `threads` per CTA: 32..256, a multiple of
-// 32 (one warp per 32 vectors).
-constexpr int kTStreamThreads = 128;   // default CTA size
+// Transposing 2D passes, chunk-delayed, the sample ring in tensor memory
+// (tring_impl.cuh): vectors with adjacent samples in, destination-major output
+// with the vectors adjacent, or (`tiled`, Float32) in tiles of 32 vectors.
+// Every job of a launch has the same window (StreamPack::ring_window) and its
+// plan view the matching records; `per_lane` vectors a lane (1 or 2), CTAs of kTRingThreads threads.
+constexpr int kTStreamThreads = 128;   // default CTA size of the two-pass kernels
+constexpr int kTRingThreads = 128;
 constexpr int kTResidentWarps = 16;    // resident warps per SM (128 registers a thread)
 constexpr int kMinSegmentChunks = 1;   // shortest segment, in chunks (StreamJob)
-int launch_tstream(const dev::StreamJob *jobs, int job_count, int total_blocks, int threads,
-                   int half_bandwidth, int window, dev::Sample in, dev::Sample out, int record_floats,
-                   void *stream);
-
-// Paired transposing 2D passes (tstream2_impl.cuh): as launch_tstream with
-// two vectors per thread (a CTA of `threads` covers 2 x threads vectors) and
-// the plans' paired records; windows <= 16.
-int launch_tstream2(const dev::StreamJob *jobs, int job_count, int total_blocks, int threads,
-                    int half_bandwidth, int window, dev::Sample in, dev::Sample out, int record_floats,
-                    void *stream);
+int launch_tring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
+                 int per_lane, bool tiled, dev::Sample in, dev::Sample out, void *stream);
 
 // Columns passes with fused candidate scoring (tscore_impl.cuh): as
-// launch_tstream for Float32 intermediates with chunk-delayed records
+// the transposing passes, for Float32 intermediates with chunk-delayed records
 // (window 0, 8, 12 or 16) and half-bandwidths 1..7, every job carrying a
 // ScoreEpilogue (score.cuh) and starting on a CTA of kScoreCtaThreads
 // threads, one CTA per tile; nothing is stored but the tiles' partials.

@@ -45,6 +45,15 @@ bool ring_fits_grouped(const std::vector<int> &s0, int window, int size, int rin
 
 } // namespace
 
+int ring_window(int half_bandwidth, int window) {
+    // Half-bandwidth 1 windows are 4 samples below a ratio of 1.5; wider
+    // kernels' never are.
+    if (half_bandwidth == 1 && window <= 4) return 4;
+    if (half_bandwidth <= 5 && window <= 8) return 8;
+    if (half_bandwidth >= 3 && window <= 12) return 12;
+    return window <= 16 ? 16 : 0;
+}
+
 StreamPack pack_stream_plan(const AxisPlan &p, int chunk, int ring, bool hb_supported, bool hb_supported_exact) {
     StreamPack out;
     const int n = p.destination_size, m = p.source_size, hb = p.half_bandwidth;
@@ -275,33 +284,47 @@ StreamPack pack_stream_plan(const AxisPlan &p, int chunk, int ring, bool hb_supp
     out.chunk_first_block.resize(static_cast<std::size_t>(chunks));
     for (int k = 0; k < chunks; ++k) out.chunk_first_block[static_cast<std::size_t>(k)] = s0[static_cast<std::size_t>(k) * chunk] / 16 * 16;
 
-    if (delayed && out.ring_ok_transposed && window <= 16) {
-        const int pl = round4(2 * hb);
-        out.paired = true;
-        out.paired_forward_stride = 4 + 2 * window + pl;
-        out.paired_backward_stride = std::max(4, pl);
-        out.paired_forward.assign(padded * static_cast<std::size_t>(out.paired_forward_stride), 0.0F);
-        out.paired_backward.assign(padded * static_cast<std::size_t>(out.paired_backward_stride), 0.0F);
-        for (std::size_t j = 0; j < padded; ++j) {
-            const float *f = out.forward.data() + j * static_cast<std::size_t>(out.forward_stride);
-            float *g = out.paired_forward.data() + j * static_cast<std::size_t>(out.paired_forward_stride);
-            g[0] = f[0];                                   // window start bits
-            g[1] = f[1];                                   // inverse diagonal, twice
-            g[2] = f[1];
-            int start = 0;                                 // ring offset in float2 units
-            std::memcpy(&start, &f[0], sizeof(int));
-            const int ring_offset = (start & (kStreamRing - 1)) * (kPairedRingPitch / 2);
-            std::memcpy(&g[3], &ring_offset, sizeof(int));
-            for (int k = 0; k < window + hb; ++k) {        // weights, then -lower
-                g[4 + 2 * k] = f[4 + k];
-                g[4 + 2 * k + 1] = f[4 + k];
+    const int rw = delayed && out.ring_ok_transposed ? ring_window(hb, window) : 0;
+    if (rw) {
+        // Replay of the refills: sixteen samples at a time, up to the end of
+        // the group's last window.  (A source shorter than the compiled
+        // window starts it at 0 and fills only what it has: the ring starts
+        // zeroed and the window's weights there are zero.)
+        auto start_of = [&](std::size_t j) { return std::min(s0[std::min(j, w - 1)], std::max(0, m - rw)); };
+        auto end_of = [&](std::size_t j) { return std::min(m, start_of(j) + rw); };
+        int have = 0, held = 0;
+        for (std::size_t g = 0; g < padded; g += 4) {
+            have = std::max(have, (end_of(g + 3) + 15) / 16 * 16);
+            held = std::max(held, have - start_of(g));
+        }
+        if (held <= kRingColumns) {
+            out.ring_window = rw;
+            const auto low_floats = static_cast<std::size_t>(round4(4 * hb));
+            const std::size_t gs = 8 + 4 * static_cast<std::size_t>(rw) + low_floats;
+            out.ring_forward.assign(padded / 4 * gs, 0.0F);
+            out.ring_backward.assign(padded / 4 * low_floats, 0.0F);
+            for (std::size_t j = 0; j < padded; ++j) {
+                float *f = out.ring_forward.data() + j / 4 * gs;
+                float *b = out.ring_backward.data() + j / 4 * low_floats;
+                const std::size_t q = j % 4, h = static_cast<std::size_t>(hb);
+                int head = start_of(j) % kRingColumns;
+                if (q == 0) head |= end_of(j + 3) << 8;
+                std::memcpy(&f[q], &head, sizeof(int));
+                const float *r = out.forward.data() + j * static_cast<std::size_t>(out.forward_stride);
+                f[4 + q] = r[1];
+                if (j < w) {
+                    const auto at = static_cast<std::size_t>(s0[j] - start_of(j));
+                    for (int k = 0; k < window; ++k)
+                        f[8 + q * static_cast<std::size_t>(rw) + at + static_cast<std::size_t>(k)] = r[4 + k];
+                }
+                for (std::size_t i = 0; i < h; ++i) {
+                    f[8 + 4 * static_cast<std::size_t>(rw) + q * h + i] = r[4 + static_cast<std::size_t>(window) + i];
+                    b[q * h + i] = out.backward[j * static_cast<std::size_t>(out.backward_stride) + i];
+                }
             }
-            const float *b = out.backward.data() + j * static_cast<std::size_t>(out.backward_stride);
-            float *h = out.paired_backward.data() + j * static_cast<std::size_t>(out.paired_backward_stride);
-            for (int q = 0; q < hb; ++q) {
-                h[2 * q] = -b[q];
-                h[2 * q + 1] = -b[q];
-            }
+            out.ring_first_block.resize(static_cast<std::size_t>(chunks));
+            for (int k = 0; k < chunks; ++k)
+                out.ring_first_block[static_cast<std::size_t>(k)] = start_of(static_cast<std::size_t>(k) * chunk) / 16 * 16;
         }
     }
     return out;

@@ -1,5 +1,5 @@
 // Host packing of an axis plan for the streaming kernels (stream_impl.cuh,
-// tstream_impl.cuh, tstream2_impl.cuh) and the checks that admit a plan.
+// tring_impl.cuh, tsolve_impl.cuh, tscore_impl.cuh) and the checks that admit a plan.
 #pragma once
 
 #include "planner.hpp"
@@ -61,15 +61,24 @@ struct StreamPack {
     // records past the end).
     std::vector<float> forward;     // * forward_stride
     std::vector<float> backward;    // * backward_stride
-    // Records of the paired 2D kernels (tstream2_impl.cuh), when the window
-    // is at most 16 and the transposing feed fits: every coefficient twice,
-    // backward factors negated.
-    bool paired = false;
-    int paired_forward_stride = 0;  // 4 + 2 window + round4(2 hb)
-    int paired_backward_stride = 0; // round4(2 hb)
-    std::vector<float> paired_forward;
-    std::vector<float> paired_backward;
+    // Records of the 2D kernels with the ring in tensor memory
+    // (tring_impl.cuh), when the plan is eligible and their feed fits: the
+    // window is ring_window(hb, window) samples, starting at most at
+    // source_size - ring_window.  Per group of four destinations: their four
+    // ring columns (start mod kRingColumns), the first word also holding the refill
+    // target (the group's last window's end) above bit 8; the four inverse
+    // diagonals; the four windows' weights; the four destinations' lower
+    // factors back to back (use order d = hb..1), padded to 4.  Backward:
+    // the four destinations' hb factors back to back, padded to 4.
+    int ring_window = 0;            // 0 when not admitted
+    std::vector<float> ring_forward;
+    std::vector<float> ring_backward;
+    std::vector<int> ring_first_block;   // as chunk_first_block, for these windows
 };
+
+// The compiled window that serves a plan's window in the kernels with the
+// ring in tensor memory; 0 when none does.
+int ring_window(int half_bandwidth, int window);
 
 // `chunk` destinations per register chunk, `ring` source samples held per
 // thread.  A plan is eligible when its half-bandwidth has a kernel, its

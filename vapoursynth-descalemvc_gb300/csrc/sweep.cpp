@@ -573,8 +573,8 @@ struct Sweep::Impl {
     void autotune() {
         const auto t0 = std::chrono::steady_clock::now();
         Wave &w = waves.front();
-        // Two right-hand sides a lane only where some plan admits the paired
-        // kernels: otherwise both batches are the same launches.
+        // Two right-hand sides a lane only where some plan runs the
+        // chunk-delayed kernels: otherwise both batches are the same launches.
         auto single = executor->prepare_batch(w.tasks, nullptr, scratch_mem.data(), scratch_capacity, 32);
         auto paired = executor->prepare_batch(w.tasks, nullptr, scratch_mem.data(), scratch_capacity, 64);
         const auto paired_groups = paired->groups();
@@ -593,8 +593,10 @@ struct Sweep::Impl {
         for (const int threads : {64, 128, 256}) {
             BatchTuning all;
             for (const auto &g : keys) {
-                const int most = g.kind >= 3 ? 256 : 128;
-                if (g.kind != 2 && g.kind <= 6 && threads <= most) all[g.key] = threads;
+                // The chunk-delayed kernels have one CTA size.
+                const bool ring = g.kind == 3 || g.kind == 4;
+                const int most = g.kind >= 3 && !ring ? 256 : 128;
+                if (g.kind != 2 && g.kind <= 6 && threads <= most && (!ring || threads == 128)) all[g.key] = threads;
             }
             if (all.empty()) continue;
             auto batch = executor->prepare_batch(w.tasks, &all, scratch_mem.data(), scratch_capacity,

@@ -1,0 +1,619 @@
+// Chunk-delayed transposing kernels with the sample ring in tensor memory:
+// the two passes of a Float32 2D descale.
+//
+// Both passes read vectors whose samples are adjacent (rows of the input
+// plane; columns of the intermediate) and write their results transposed,
+// destination-major with the vectors adjacent.  A lane owns V vectors, a warp
+// 32 V.
+//
+//  * Loads: blocks of 128 bytes of every vector of the warp come by TMA (one
+//    tensor map per plane, 128-byte swizzle) into one of the warp's two
+//    staging buffers, completed on that buffer's mbarrier; the next block is
+//    in flight while the current one is consumed.  The swizzle lets a lane
+//    read its own vectors without bank conflicts.  Every wait is bounded.
+//  * Ring: a lane converts 16 samples of its vectors at a time to float and
+//    stores them to tensor memory (lane = vector, column = sample mod 48, the
+//    first 16 columns again after the ring so that every window of up to 16
+//    is contiguous).  A destination's window is then one load at a column
+//    that is known only at run time: tensor memory serves as a register file
+//    that can be indexed, at about 1.3 SM cycles for 8 columns of a warp,
+//    where shared memory takes 8 (and the sample scatter 1.5 a sample).
+//  * Forward values: also in tensor memory, two chunks a vector, so that the
+//    substitutions are loops over groups of destinations instead of 32
+//    unrolled destinations on 64 registers of forward values; ring and
+//    forward values are 128 columns, four CTAs of one vector a lane an SM.
+//  * Intermediate: in tiles of 32 rows, [row / 32][destination][row mod 32]:
+//    the first pass stores at constant offsets, the second reads 128
+//    contiguous bytes of each vector.
+//  * Records: copied (cp.async) a chunk of 32 destinations at a time, three
+//    deep, for the CTA's four warps.  A warp-wide load of the same 16 bytes
+//    takes two shared-memory cycles, which is what two vectors a lane save.
+//  * Arithmetic: exact forward substitution (the gather's even and odd taps
+//    in two sums), chunk-delayed backward substitution with a zero-carry
+//    warm-up over the following chunk.  Every rounding is the same for any V.
+//
+// What bounds them: instruction issue (53 instructions per 32 results at one
+// vector a lane, 0.62 of the issue slots busy) beside the shared-memory pipe
+// (14.5 cycles per 32 results, 61 % busy).  Measured on one GB300 against the
+// kernels with both in registers and shared memory: 64 YUV420P16 1080p frames
+// to 810p 769 -> 536 us, 32 4K Float32 frames to 1440p 1017 -> 604 us.
+#pragma once
+
+#include "tstream_impl.cuh"
+
+namespace dsmvc_gb {
+namespace {
+
+constexpr int kRingThreads = 128;            // four warps: one per tensor-memory lane quarter
+constexpr int kRingStep = 16;                // samples converted at a time
+// try_wait rounds before a feed wait gives up, each suspending at most
+// kFeedWaitSuspendNs (about 65 ms in all, far beyond any copy's latency); a
+// stalled warp stops waiting and its kernel reports kStatusFeedStall.
+constexpr int kFeedWaitRounds = 1 << 16;
+constexpr unsigned kFeedWaitSuspendNs = 1000;
+constexpr int kRingBuffers = 2;              // staged blocks: one consumed, the others in flight
+
+// ---- tensor memory -----------------------------------------------------------
+
+__device__ __forceinline__ void tm_ld4(float *x, unsigned a) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(a));
+}
+__device__ __forceinline__ void tm_ld8(float *x, unsigned a) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7])
+                 : "r"(a));
+}
+__device__ __forceinline__ void tm_st8(unsigned a, const float *x) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"
+                 :: "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]), "f"(x[4]), "f"(x[5]), "f"(x[6]), "f"(x[7]), "r"(a));
+}
+__device__ __forceinline__ void tm_st4(unsigned a, const float *x) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%4], {%0,%1,%2,%3};"
+                 :: "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]), "r"(a));
+}
+__device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;"); }
+template <int N> __device__ __forceinline__ void tm_ld(float *x, unsigned a) {
+#pragma unroll
+    for (int i = 0; i + 8 <= N; i += 8) tm_ld8(x + i, a + i);
+    if constexpr (N % 8) tm_ld4(x + N / 8 * 8, a + N / 8 * 8);
+}
+// Every load issued so far has arrived; no use of x moves before this.
+template <int N> __device__ __forceinline__ void tm_pin(float *x) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4)
+        asm volatile("" : "+f"(x[i]), "+f"(x[i + 1]), "+f"(x[i + 2]), "+f"(x[i + 3]));
+}
+__device__ __forceinline__ void tm_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;"); }
+
+// Output samples: rounding before the clamp to [0, out_max] gives what the
+// clamp before it does (the bounds are whole, the conversion saturates below
+// at 0 and NaN converts to 0).
+template <class T> __device__ __forceinline__ T rout(float v, const Conversion &c) {
+    if constexpr (sizeof(T) == 4) return v;
+    else return static_cast<T>(min(__float2uint_rn(__fadd_rn(__fmul_rn(v, c.out_scale), c.out_offset)), c.out_max));
+}
+
+// ---- ring feeder ---------------------------------------------------------------
+
+template <class In, int V, int W>
+struct RingFeeder {
+    static constexpr int SPL = 16 / static_cast<int>(sizeof(In));   // samples per 16 bytes
+    static constexpr int SB = 8 * SPL;                              // samples per staged block
+    static constexpr int DUP = W <= 8 ? 8 : 16;                     // columns stored again after the ring
+    static constexpr int VC = kRingColumns + 16;                    // columns per vector
+    static constexpr int BUFFER = 32 * V * 128;                     // bytes per staging buffer
+    static constexpr int NR = kRingStep * static_cast<int>(sizeof(In)) / 4;   // words of a step's samples
+
+    const void *in;          // the plane
+    std::int64_t in_vec;
+    std::uint64_t map;       // its tensor map, 0: vectors not 16-byte aligned
+    int first;               // the warp's first vector
+    int vectors;             // its valid vectors (>= 1)
+    int size;                // samples per vector
+    int limit;               // blocks that start before this sample are fetched
+    int lane;
+    unsigned ring;           // tensor-memory address of the warp's ring
+    unsigned stage;          // staging buffers of this warp (shared address)
+    unsigned mbar;           // their barriers (8 bytes apart)
+    unsigned row[V];         // this lane's vectors in a staging buffer (byte offset)
+    float in_offset, in_scale;
+    int have;                // samples in the ring (a multiple of 16)
+    int column;              // have mod kRingColumns
+    int next;                // sample where the next block to fetch starts
+    int count;               // blocks consumed or being consumed
+    unsigned at;             // the block being consumed (shared address)
+    bool tiled;
+    bool failed;             // a wait ran out: nothing more is fetched or waited for
+
+    // Fetches the block at `next` into buffer `slot`.
+    __device__ __forceinline__ void issue(unsigned slot) {
+        unsigned elected;
+        asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(elected));
+        if (elected && next < limit) {
+            const unsigned mb = mbar + slot * 8;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" :: "r"(mb), "r"(BUFFER) : "memory");
+            asm volatile("cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes"
+                         " [%0], [%1, {%2, %3, %4}], [%5];\n"
+                         :: "r"(stage + slot * BUFFER), "l"(map), "r"(tiled ? 0 : next), "r"(first),
+                            "r"(tiled ? next / 32 : 0), "r"(mb) : "memory");
+        }
+        next += SB;
+    }
+
+    __device__ __forceinline__ bool arrived(int k) const {
+        unsigned done;
+        asm volatile("{\n .reg .pred q;\n mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2, %3;\n"
+                     " selp.u32 %0, 1, 0, q;\n}\n"
+                     : "=r"(done) : "r"(mbar + (k & 1) * 8), "r"(k >> 1 & 1), "r"(kFeedWaitSuspendNs) : "memory");
+        return done;
+    }
+
+    // Waits, within a limit, for the k-th block's copy.
+    __device__ __noinline__ bool wait(int k) const {
+        for (int it = 0; it < kFeedWaitRounds; ++it)
+            if (arrived(k)) return true;
+        return false;
+    }
+
+    // Enters the next block; the one after it goes to the other buffer, which
+    // every lane has read.
+    __device__ __forceinline__ void enter() {
+        if (!arrived(count) && !failed && !wait(count)) {
+            failed = true;
+            limit = 0;
+        }
+        at = stage + (count & 1) * BUFFER;
+        ++count;
+        __syncwarp();
+        issue(count & 1);
+    }
+
+    // Waits for the copies still in flight (the block being consumed and the
+    // next): none writes to shared memory after the CTA has ended.
+    __device__ __forceinline__ void drain() const {
+        if (map)
+            for (int k = max(count - 1, 0), from = next - (count - k + 1) * SB; k <= count; ++k, from += SB)
+                if (from < size) wait(k);
+    }
+
+    // Loads the next step's samples of every vector.
+    __device__ __forceinline__ void fetch(unsigned (&raw)[V][NR]) {
+        if (map) {
+            if (have % SB == 0) enter();
+            // 16-byte pieces lie in the tensor map's 128-byte swizzle.
+            const unsigned piece = (have % SB) / SPL;
+#pragma unroll
+            for (int a = 0; a < V; ++a) {
+#pragma unroll
+                for (int i = 0; i < NR / 4; ++i)
+                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(raw[a][4 * i]), "=r"(raw[a][4 * i + 1]), "=r"(raw[a][4 * i + 2]),
+                                   "=r"(raw[a][4 * i + 3])
+                                 : "r"(at + (row[a] ^ ((piece + i) * 16))));
+            }
+        } else {
+            // Vectors that no tensor map admits (not 16-byte aligned): each
+            // lane loads its own.
+#pragma unroll
+            for (int a = 0; a < V; ++a) {
+                const In *p = static_cast<const In *>(in) + (first + min(lane + 32 * a, vectors - 1)) * in_vec;
+                In vals[kRingStep];
+#pragma unroll
+                for (int i = 0; i < kRingStep; ++i) vals[i] = __ldg(p + min(have + i, size - 1));
+#pragma unroll
+                for (int i = 0; i < NR; ++i) {
+                    unsigned w = 0;
+                    if constexpr (sizeof(In) == 4) {
+                        w = __float_as_uint(vals[i]);
+                    } else {
+                        constexpr int N = 4 / static_cast<int>(sizeof(In));
+#pragma unroll
+                        for (int k = 0; k < N; ++k) w |= static_cast<unsigned>(vals[i * N + k]) << (k * 32 / N);
+                    }
+                    raw[a][i] = w;
+                }
+            }
+        }
+    }
+
+    // `from`: a multiple of 16 at most the first window start.
+    __device__ __forceinline__ void start(int from) {
+        const float zero[8] = {};
+        for (int c = 0; c < V * VC; c += 8) tm_st8(ring + c, zero);
+        tm_wait_st();
+        have = from;
+        column = from % kRingColumns;
+        count = 0;
+        next = from / SB * SB;
+        if (map) {
+            issue(0);
+            if (from % SB) enter();
+        }
+    }
+
+    // The next 16 samples of every vector.
+    __device__ __forceinline__ void step() {
+        unsigned raw[V][NR];
+        fetch(raw);
+#pragma unroll
+        for (int a = 0; a < V; ++a) {
+            float f[kRingStep];
+            if constexpr (sizeof(In) == 4) {
+#pragma unroll
+                for (int i = 0; i < kRingStep; ++i) f[i] = __uint_as_float(raw[a][i]);
+            } else {
+                const In *vals = reinterpret_cast<const In *>(raw[a]);
+                const float2 off = make_float2(-in_offset, -in_offset), scale = make_float2(in_scale, in_scale);
+#pragma unroll
+                for (int i = 0; i < kRingStep; i += 2) {
+                    const float2 v = make_float2(static_cast<float>(vals[i]), static_cast<float>(vals[i + 1]));
+                    const float2 r = __fmul2_rn(__fadd2_rn(v, off), scale);
+                    f[i] = r.x;
+                    f[i + 1] = r.y;
+                }
+            }
+            const unsigned to = ring + a * VC + column;
+            // The ring's first columns are stored again after it (other
+            // steps store theirs twice).
+            const unsigned dup = column ? to : to + kRingColumns;
+#pragma unroll
+            for (int i = 0; i < kRingStep; i += 4) {
+                tm_st4(to + i, f + i);
+                if (i < DUP) tm_st4(dup + i, f + i);
+            }
+        }
+        have += kRingStep;
+        column = column + kRingStep == kRingColumns ? 0 : column + kRingStep;
+    }
+
+    // Makes samples [0, need) resident (need <= size).
+    __device__ __forceinline__ void ensure(int need) {
+        if (have >= need) return;
+        do step(); while (have < need);
+        tm_wait_st();
+    }
+};
+
+// ---- records ---------------------------------------------------------------------
+
+// Records (StreamPack::ring_forward, ring_backward): per group of four
+// destinations, four ring columns (the first word also holds the refill
+// target above bit 8), the four inverse diagonals, the four windows' weights,
+// and the four destinations' lower factors back to back; the four
+// destinations' backward factors back to back.
+template <int HB, int W> struct RingRecord {
+    static constexpr int LOW = 4 * HB;
+    static constexpr int GROUP = 8 + 4 * W + LOW;     // floats per group
+    static constexpr int GROUPS = kTChunk / 4;
+    static constexpr int CHUNK = GROUPS * (GROUP + LOW);
+};
+
+// ---- substitutions ---------------------------------------------------------------
+
+// Destinations per iteration of the substitution loops (each iteration moves
+// its histories; one vector a lane spills with more).
+template <int V> constexpr int kRingGroup = V == 2 ? 16 : 8;
+
+template <int N> __device__ __forceinline__ void rload(float (&c)[N], const float *from) {
+    static_assert(N % 4 == 0);
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+        const float4 l = tlds4(from + i);
+        c[i] = l.x;
+        c[i + 1] = l.y;
+        c[i + 2] = l.z;
+        c[i + 3] = l.w;
+    }
+}
+
+// Forward substitution of a chunk: its values to tensor memory at `ycol`
+// (column = destination of the chunk, a lane's vectors 64 columns apart).
+// `hist`: the HB values before it, oldest first.
+template <int HB, int W, int V, class Feed>
+__device__ __forceinline__ void rforward(float (&hist)[V][HB], const float *fwd, unsigned ycol, Feed &feed) {
+    using R = RingRecord<HB, W>;
+    constexpr int G = kRingGroup<V>;
+#pragma unroll 1
+    for (int tg = 0; tg < kTChunk; tg += G) {
+        float y[V][HB + G];                               // y[HB + t]: destination tg + t
+#pragma unroll
+        for (int a = 0; a < V; ++a)
+#pragma unroll
+            for (int d = 0; d < HB; ++d) y[a][d] = hist[a][d];
+#pragma unroll
+        for (int t = 0; t < G; t += 4) {
+            const float *gr = fwd + ((tg + t) / 4) * R::GROUP;
+            const int4 h = *reinterpret_cast<const int4 *>(gr);
+            feed.ensure(h.x >> 8);
+            const unsigned at[4] = {feed.ring + (h.x & 255), feed.ring + h.y, feed.ring + h.z, feed.ring + h.w};
+            float x[2][V][W];
+#pragma unroll
+            for (int a = 0; a < V; ++a) tm_ld<W>(x[0][a], at[0] + a * Feed::VC);
+            float iv[4], lw[R::LOW];
+            rload(iv, gr + 4);
+            rload(lw, gr + 8 + 4 * W);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                tm_wait_ld();
+#pragma unroll
+                for (int a = 0; a < V; ++a) tm_pin<W>(x[q & 1][a]);
+                if (q < 3) {
+#pragma unroll
+                    for (int a = 0; a < V; ++a) tm_ld<W>(x[(q + 1) & 1][a], at[(q + 1) & 3] + a * Feed::VC);
+                }
+                // Even and odd taps in the two halves, then their sum.
+                float2 acc[V];
+#pragma unroll
+                for (int a = 0; a < V; ++a) acc[a] = make_float2(0.0f, 0.0f);
+#pragma unroll
+                for (int i = 0; i < W; i += 4) {
+                    const float4 w = tlds4(gr + 8 + q * W + i);
+#pragma unroll
+                    for (int a = 0; a < V; ++a) {
+                        const float *xa = x[q & 1][a] + i;
+                        acc[a] = __ffma2_rn(make_float2(w.x, w.y), make_float2(xa[0], xa[1]), acc[a]);
+                        acc[a] = __ffma2_rn(make_float2(w.z, w.w), make_float2(xa[2], xa[3]), acc[a]);
+                    }
+                }
+#pragma unroll
+                for (int a = 0; a < V; ++a) {
+                    float sum = acc[a].x + acc[a].y;
+#pragma unroll
+                    for (int e = 0; e < HB; ++e) sum = fmaf(lw[q * HB + e], y[a][t + q + e], sum);
+                    // Records past the end of the vector are zero (inverse
+                    // diagonal included): their forward values are zero.
+                    y[a][HB + t + q] = sum * iv[q];
+                }
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < V; ++a) {
+#pragma unroll
+            for (int t = 0; t < G; t += 8) tm_st8(ycol + a * 2 * kTChunk + tg + t, &y[a][HB + t]);
+#pragma unroll
+            for (int d = 0; d < HB; ++d) hist[a][d] = y[a][G + d];
+        }
+    }
+    tm_wait_st();
+}
+
+// Backward substitution of a chunk from its forward values at `ycol` and the
+// HB results after it, `carry` (nearest first; the chunk's first HB results
+// on return).  MODE 0: the warm-up, nothing stored; 1: every result stored as
+// soon as it is known; 2: those of the chunk's first `valid` destinations.
+// `at`: the chunk's first destination; STEP: the output's destination stride,
+// 0: `out_elem`.
+template <int HB, int W, int V, int MODE, int STEP, class Out>
+__device__ __forceinline__ void rbackward(float (&carry)[V][HB], const float *bwd, unsigned ycol, int valid,
+                                          Out *const (&out)[V], std::int64_t at, std::int64_t out_elem,
+                                          const Conversion &conv) {
+    using R = RingRecord<HB, W>;
+    constexpr int G = kRingGroup<V>;
+#pragma unroll 1
+    for (int tg = kTChunk - G; tg >= 0; tg -= G) {
+        float y[V][G], x[V][G + HB];
+#pragma unroll
+        for (int a = 0; a < V; ++a)
+#pragma unroll
+            for (int t = 0; t < G; t += 8) tm_ld8(&y[a][t], ycol + a * 2 * kTChunk + tg + t);
+#pragma unroll
+        for (int a = 0; a < V; ++a)
+#pragma unroll
+            for (int d = 0; d < HB; ++d) x[a][G + d] = carry[a][d];
+        Out *o[V];
+        if constexpr (MODE > 0) {
+#pragma unroll
+            for (int a = 0; a < V; ++a) o[a] = out[a] + (STEP ? (at + tg) * STEP : (at + tg + G - 1) * out_elem);
+        }
+        float u[2][R::LOW];
+        rload(u[(G / 4 - 1) & 1], bwd + (tg / 4 + G / 4 - 1) * R::LOW);
+        tm_wait_ld();
+#pragma unroll
+        for (int a = 0; a < V; ++a) tm_pin<G>(y[a]);
+#pragma unroll
+        for (int t = G - 1; t >= 0; --t) {
+            if (t % 4 == 3 && t > 4) rload(u[(t / 4 - 1) & 1], bwd + (tg / 4 + t / 4 - 1) * R::LOW);
+#pragma unroll
+            for (int a = 0; a < V; ++a) {
+                float sum = 0.0f;
+#pragma unroll
+                for (int pos = 0; pos < HB; ++pos)
+                    sum = fmaf(u[(t / 4) & 1][(t % 4) * HB + pos], x[a][t + (HB == 3 ? pos + 1 : HB - pos)], sum);
+                x[a][t] = y[a][t] - sum;
+                if constexpr (MODE > 0) {
+                    Out *to = STEP ? o[a] + t * STEP : o[a];
+                    if (MODE == 1 || tg + t < valid) *to = rout<Out>(x[a][t], conv);
+                    if constexpr (STEP == 0) o[a] -= out_elem;
+                }
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < V; ++a)
+#pragma unroll
+            for (int d = 0; d < HB; ++d) carry[a][d] = x[a][d];
+    }
+}
+
+// TILED: the output is the intermediate in tiles of 32 vectors,
+// [vector / 32][destination][vector mod 32].
+template <int HB, int W, int V, bool TILED, class In, class Out>
+__global__ void __launch_bounds__(kRingThreads, 4 / V)
+tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
+    using R = RingRecord<HB, W>;
+    using Feed = RingFeeder<In, V, W>;
+    constexpr int LC = kTChunk, WARPS = kRingThreads / 32, STEP = TILED ? 32 : 0;
+    constexpr int COLUMNS = 128 * V;       // the rings and two chunks of forward values
+    static_assert(V * (Feed::VC + 2 * LC) <= COLUMNS);
+    // Staging buffers (WARPS * kRingBuffers of Feed::BUFFER bytes, where the
+    // 128-byte swizzle's pattern of 1024 begins), then three chunks of records.
+    extern __shared__ unsigned char ring_dynamic[];
+    unsigned char *const ring_smem = ring_dynamic + (-static_cast<unsigned>(__cvta_generic_to_shared(ring_dynamic)) & 1023);
+    float *bufs = reinterpret_cast<float *>(ring_smem + WARPS * kRingBuffers * Feed::BUFFER);
+    __shared__ unsigned long long feed_bar[WARPS][kRingBuffers];
+    __shared__ unsigned tm_base;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // Jobs are assigned warps; a CTA's warps share one plan and one chunk
+    // range (the host rounds changes of either up to whole CTAs), whose
+    // records the CTA copies once.
+    const int cta_warp = static_cast<int>(blockIdx.x) * WARPS;
+    const StreamJob &job = jobs[find_tjob(jobs, job_count, cta_warp + warp)];
+    const StreamJob &lead = jobs[find_tjob(jobs, job_count, cta_warp)];
+    const dev::StreamPlanView p = lead.plan;
+    const int n = p.destination_size;
+    const int chunks = (n + LC - 1) / LC;
+    // Chunks whose outputs this CTA stores: [ca, cb).  The forward
+    // substitution runs over [c0, ce]: from one chunk early (zero history)
+    // for a range past chunk 0, to one chunk late (the backward warm-up of
+    // the last stored chunk) for a range ending before the last chunk.
+    const int ca = lead.chunk_begin;
+    const int cb = lead.chunk_end > 0 ? lead.chunk_end : chunks;
+    const int c0 = ca > 0 ? ca - 1 : 0;
+    const int ce = cb < chunks ? cb : chunks - 1;
+
+    tstage(bufs + (c0 % 3) * R::CHUNK, p, c0, tid, kRingThreads);
+    tcp_commit();
+    if (c0 + 1 <= ce) tstage(bufs + ((c0 + 1) % 3) * R::CHUNK, p, c0 + 1, tid, kRingThreads);
+    tcp_commit();
+
+    if (warp == 0) {
+        // The allocation ends: a CTA waiting for it holds none, and those that
+        // hold theirs wait for nothing of another CTA's.
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
+                     :: "r"(static_cast<unsigned>(__cvta_generic_to_shared(&tm_base))), "n"(COLUMNS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+    }
+    if (lane < kRingBuffers) {
+        const unsigned mb = static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][lane]));
+        // A stall test expects an arrival that nothing makes.
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" :: "r"(mb), "r"(lead.feed_stall_test ? 2 : 1) : "memory");
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;\n");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n");
+
+    // The warp's vectors; a warp past its job's last vector only takes part
+    // in the CTA's record copies and barriers.
+    const int warp_first = (cta_warp + warp - job.first_block) * 32 * V;
+    const int left = job.vectors - warp_first;
+    const bool idle = left <= 0;
+    const unsigned tm = tm_base;
+    Feed feed;
+    feed.in = job.in;
+    feed.in_vec = job.in_vec;
+    feed.map = job.mapped ? reinterpret_cast<std::uint64_t>(job.map) : 0;
+    feed.first = idle ? 0 : warp_first;
+    feed.vectors = idle ? 1 : left > 32 * V ? 32 * V : left;
+    feed.size = feed.limit = p.source_size;
+    feed.lane = lane;
+    feed.ring = tm + (static_cast<unsigned>(warp * 32) << 16);
+    feed.stage = static_cast<unsigned>(__cvta_generic_to_shared(ring_smem + warp * kRingBuffers * Feed::BUFFER));
+    feed.mbar = static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][0]));
+    // Lanes past the warp's last vector repeat it: same samples, same results,
+    // stored to the same place.
+#pragma unroll
+    for (int a = 0; a < V; ++a) {
+        const unsigned v = min(lane + 32 * a, feed.vectors - 1);
+        feed.row[a] = v * 128 + (v & 7) * 16;
+    }
+    feed.in_offset = job.conv.in_offset;
+    feed.in_scale = job.conv.in_scale;
+    feed.tiled = job.mapped == 2;
+    feed.failed = false;
+    if (feed.map && lane == 0)
+        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" :: "l"(feed.map) : "memory");
+    __syncwarp();
+    if (!idle) feed.start(c0 > 0 ? lead.first_sample : 0);
+
+    Out *out[V];
+#pragma unroll
+    for (int a = 0; a < V; ++a) {
+        const int v = idle ? 0 : warp_first + min(lane + 32 * a, feed.vectors - 1);
+        out[a] = static_cast<Out *>(job.out) + (TILED ? static_cast<std::int64_t>(v >> 5) * n * 32 + (v & 31) : v);
+    }
+
+    const Conversion conv = job.conv;
+    const std::int64_t out_elem = job.out_elem;
+    const unsigned ycol = feed.ring + V * Feed::VC;        // chunk c's forward values 32 (c & 1) columns on
+    float hist[V][HB], carry[V][HB];
+#pragma unroll
+    for (int a = 0; a < V; ++a)
+#pragma unroll
+        for (int d = 0; d < HB; ++d) hist[a][d] = 0.0f;
+    for (int c = c0;; ++c) {
+        tcp_wait_one();
+        __syncthreads();
+        const float *cur = bufs + (c % 3) * R::CHUNK;
+        float *prev = bufs + ((c + 2) % 3) * R::CHUNK;
+        if (!idle) {
+            const unsigned yc = ycol + (c & 1) * LC, yp = ycol + (~c & 1) * LC;
+            rforward<HB, W, V>(hist, cur, yc, feed);
+            const float *cur_b = cur + R::GROUPS * R::GROUP;
+#pragma unroll
+            for (int a = 0; a < V; ++a)
+#pragma unroll
+                for (int d = 0; d < HB; ++d) carry[a][d] = 0.0f;
+            if (c + 1 == chunks) {
+                // The vector's last chunk: exact from the end, stored when the
+                // chunk is the CTA's.
+                rbackward<HB, W, V, 2, STEP>(carry, cur_b, yc, c < cb ? n - c * LC : 0, out, c * LC, out_elem, conv);
+            } else if (c > ca) {
+                rbackward<HB, W, V, 0, STEP>(carry, cur_b, yc, 0, out, 0, out_elem, conv);
+            }
+            if (c > ca)
+                rbackward<HB, W, V, 1, STEP>(carry, prev + R::GROUPS * R::GROUP, yp, LC, out, (c - 1) * LC, out_elem, conv);
+        }
+        if (c == ce) break;
+        // Every warp is done with chunk c-1's records: fetch chunk c+2.
+        __syncthreads();
+        if (c + 2 <= ce) tstage(prev, p, c + 2, tid, kRingThreads);
+        tcp_commit();
+    }
+    // No copy is left in flight; a stalled feed wait reports.
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    if (!idle) feed.drain();
+    if (__any_sync(0xffffffffu, feed.failed) && lane == 0) atomicOr(lead.status, dev::kStatusFeedStall);
+    asm volatile("tcgen05.fence::before_thread_sync;\n");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" :: "r"(tm), "n"(COLUMNS));
+}
+
+template <int HB, int W, int V, bool TILED, class In, class Out>
+int rlaunch_typed(const StreamJob *jobs, int count, int blocks, cudaStream_t s) {
+    constexpr int smem = 1024 + 3 * RingRecord<HB, W>::CHUNK * 4
+        + kRingThreads / 32 * kRingBuffers * RingFeeder<In, V, W>::BUFFER;
+    auto kernel = tring_kernel<HB, W, V, TILED, In, Out>;
+    static SmemLimit limit;
+    if (const cudaError_t e = limit.ensure(kernel, smem); e != cudaSuccess) return static_cast<int>(e);
+    kernel<<<blocks, kRingThreads, smem, s>>>(jobs, count);
+    return static_cast<int>(cudaGetLastError());
+}
+
+template <int HB, int W, int V>
+int rlaunch(const StreamJob *jobs, int count, int blocks, dev::Sample in, dev::Sample out, bool tiled, void *stream) {
+    using dev::Sample;
+    using std::uint16_t, std::uint8_t;
+    const auto s = static_cast<cudaStream_t>(stream);
+    if (out == Sample::f32) {
+        if (in == Sample::f32)
+            return tiled ? rlaunch_typed<HB, W, V, true, float, float>(jobs, count, blocks, s)
+                         : rlaunch_typed<HB, W, V, false, float, float>(jobs, count, blocks, s);
+        if (in == Sample::u16)
+            return tiled ? rlaunch_typed<HB, W, V, true, uint16_t, float>(jobs, count, blocks, s)
+                         : rlaunch_typed<HB, W, V, false, uint16_t, float>(jobs, count, blocks, s);
+        if (in == Sample::u8)
+            return tiled ? rlaunch_typed<HB, W, V, true, uint8_t, float>(jobs, count, blocks, s)
+                         : rlaunch_typed<HB, W, V, false, uint8_t, float>(jobs, count, blocks, s);
+    }
+    if (in == Sample::f32 && out == Sample::u16)
+        return rlaunch_typed<HB, W, V, false, float, uint16_t>(jobs, count, blocks, s);
+    if (in == Sample::f32 && out == Sample::u8)
+        return rlaunch_typed<HB, W, V, false, float, uint8_t>(jobs, count, blocks, s);
+    return static_cast<int>(cudaErrorInvalidValue);
+}
+
+} // namespace
+} // namespace dsmvc_gb
