@@ -368,7 +368,7 @@ int dsmvc_gb_batch_info(const dsmvc_gb_batch *batch, int64_t *kernel_launches,
  * `stream` and on a stream of the batch forked from it and joined back to it
  * (stream-ordered, capturable), so that one half's second pass overlaps the
  * other's first; 0 (what dsmvc_gb_batch_create does) chooses 2 for 8 tasks
- * or more.  dsmvc_gb_batch_parts reports the count. */
+ * of two axes or more.  dsmvc_gb_batch_parts reports the count. */
 int dsmvc_gb_batch_create_parts(dsmvc_gb_executor *executor,
                                 const dsmvc_gb_plane_task *tasks, int32_t count,
                                 int32_t parts, dsmvc_gb_batch **out);

@@ -73,3 +73,26 @@ def test_unaligned_and_paired_batches(gb, whole_executor, sample):
         for x, out in zip(planes, outs):
             got = out.cpu().numpy().view(dtype)
             assert np.array_equal(got, whole_executor.inverse_2d(h, v, x, conv if sample != "f32" else None))
+
+
+@pytest.mark.parametrize("vectors,size", [(31, 66), (33, 515), (100, 1301), (129, 1024)])
+@pytest.mark.parametrize("kernel,taps,ratio", PLANS)
+def test_one_axis(gb, executor, whole_executor, kernel, taps, ratio, vectors, size):
+    """One-axis passes: within the streaming kernels' tolerance (4e-7 of the
+    largest magnitude, test_gpu_parity.py) of the reference CUDA order, and the
+    same bits in segments as in whole vectors; rows whose pitch no tensor map
+    admits alike."""
+    h, _, oh, _ = pair(gb, kernel, taps, ratio, size, 64)
+    x = make_input(vectors, size, "f32", 5)
+    want = O.inverse_rows_gpu_order(oh, x)
+    whole = whole_executor.inverse_rows(h, x)
+    assert np.max(np.abs(whole - want)) <= 4e-7 * np.max(np.abs(want))
+    assert np.array_equal(whole, executor.inverse_rows(h, x))
+    wide = np.zeros((vectors, -(-size // 4) * 4 + 4), np.float32)
+    wide[:, :size] = x
+    out = np.zeros((vectors, -(-h.destination_size // 4) * 4 + 8), np.float32)
+    assert np.array_equal(whole, executor.inverse_rows(h, wide[:, :size], out[:, :h.destination_size]))
+    assert not out[:, h.destination_size:].any()
+    columns = whole_executor.inverse_columns(h, np.ascontiguousarray(x.T))
+    assert np.array_equal(columns, executor.inverse_columns(h, np.ascontiguousarray(x.T)))
+    assert np.max(np.abs(columns.T - want)) <= 4e-7 * np.max(np.abs(want))

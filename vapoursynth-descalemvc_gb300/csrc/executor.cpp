@@ -48,7 +48,7 @@ void cuda_check(int e, const char *what) { cuda_check(static_cast<cudaError_t>(e
 
 constexpr std::size_t kAlign = 256;
 constexpr int kSeqThreads = 128;   // threads per block of the sequential kernels
-// Prepared batches of at least this many tasks (and their own scratch) run
+// Prepared batches of at least this many 2D tasks (and their own scratch) run
 // as two parts on two streams.
 constexpr std::size_t kSplitBatchTasks = 8;
 std::size_t align_up(std::size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
@@ -751,9 +751,15 @@ int compiled_window(const DevicePlan &dp, int kind) {
 // 604; 24 YUV420P8 720x480 frames (4) 95.6 and 132.
 constexpr int kPairingWarps = 8;
 
-// The chunk-delayed transposing kinds: 3, whose vectors a lane compile()
-// chooses, and 4, two.
-bool ring_kind(int kind) { return kind == 3 || kind == 4; }
+// One-axis passes in segments: two chunks of zero-history warm-up leave below
+// 2^-52 of it, so that a segment's forward values come to the whole vector's
+// own bits.  Ranges of at least three chunks (two cost two 1080p planes 2 us of
+// 25 in repeated work; four cost one plane 2 of 21 in latency).
+constexpr int kAxisMargin = 2, kAxisMinChunks = 3;
+
+// The kinds with the ring in tensor memory: the 2D passes' 3, whose vectors a
+// lane compile() chooses, and 4, two; 10, one-axis passes.
+bool ring_kind(int kind) { return kind == 3 || kind == 4 || kind == 10; }
 
 std::string kernel_name(const GroupKey &k);
 
@@ -772,7 +778,8 @@ namespace {
 
 std::string kernel_name(const GroupKey &k) {
     static const char *kinds[] = {"axis_f32", "axis_f64", "stream_f32", "tstream_f32", "tstream2_f32",
-                                  "tsolve_f32", "tsolve_f64", "refine_f64", "convert_f64", "tscore_f32"};
+                                  "tsolve_f32", "tsolve_f64", "refine_f64", "convert_f64", "tscore_f32",
+                                  "stream_f32"};
     return std::string(kinds[k.kind]) + (k.pass ? "/columns" : "/rows") + "/hb" + std::to_string(k.hb);
 }
 
@@ -830,7 +837,8 @@ void push_segments(std::vector<Item> &group, const Item &whole, const std::vecto
 // whose forward warm-up is admitted split.  Per plan, the jobs come segment
 // by segment, so that only plan and segment changes round up to whole CTAs.
 template <class Item>
-std::vector<Item> segment_items(const std::vector<Item> &items, int vectors_per_warp, int mode, int slots) {
+std::vector<Item> segment_items(const std::vector<Item> &items, int vectors_per_warp, int mode, int slots, int margin = 1,
+                                int shortest = kMinSegmentChunks) {
     if (mode == 1) return items;
     int segments = mode;
     if (mode == 0) {
@@ -847,7 +855,7 @@ std::vector<Item> segment_items(const std::vector<Item> &items, int vectors_per_
         while (j < items.size() && items[j].stream.plan.forward == items[i].stream.plan.forward) ++j;
         const DevicePlan *dp = items[i].plan;
         const int chunks = (items[i].stream.plan.destination_size + kStreamChunk - 1) / kStreamChunk;
-        const int s = dp && dp->stream_seg ? std::max(1, std::min(segments, chunks / kMinSegmentChunks)) : 1;
+        const int s = dp && dp->stream_seg ? std::max(1, std::min(segments, chunks / shortest)) : 1;
         for (int k = 0; k < s; ++k) {
             const int begin = static_cast<int>(static_cast<long>(k) * chunks / s);
             const int end = static_cast<int>(static_cast<long>(k + 1) * chunks / s);
@@ -856,7 +864,8 @@ std::vector<Item> segment_items(const std::vector<Item> &items, int vectors_per_
                 if (s > 1) {
                     it.stream.chunk_begin = begin;
                     it.stream.chunk_end = end;
-                    it.stream.first_sample = begin > 0 ? dp->ring_first_block[static_cast<std::size_t>(begin - 1)] : 0;
+                    it.stream.margin = margin;
+                    it.stream.first_sample = dp->ring_first_block[static_cast<std::size_t>(std::max(begin - margin, 0))];
                 }
                 out.push_back(it);
             }
@@ -1225,12 +1234,15 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
             if (!v) it.bytes += static_cast<std::uint64_t>(vectors) * h->destination_size * 4;
             if (r.h_stream) {
                 auto &j = it.stream;
-                j.plan = r.h->stream_view;
+                const bool on_ring = !v && r.h->ring_window;
+                j.plan = on_ring ? r.h->ring_view : r.h->stream_view;
                 j.in = in; j.in_elem = 1; j.in_vec = in_vec;
                 j.out = out; j.out_elem = 1; j.out_vec = out_vec;
                 j.vectors = vectors;
                 j.conv = conv;
-                groups[{0, 2, h->half_bandwidth, task.sample, out_kind}].push_back(it);
+                it.plan = r.h;
+                groups[{0, on_ring ? 10 : 2, h->half_bandwidth, task.sample, out_kind, on_ring ? r.h->ring_window : 0}]
+                    .push_back(it);
             } else {
                 auto &j = it.axis;
                 j.plan = r.h->view;
@@ -1258,12 +1270,15 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
             if (!h) it.bytes += static_cast<std::uint64_t>(vectors) * v->source_size * 4;
             if (r.v_stream) {
                 auto &j = it.stream;
-                j.plan = r.v->stream_view;
+                const bool on_ring = !h && r.v->ring_window;
+                j.plan = on_ring ? r.v->ring_view : r.v->stream_view;
                 j.in = in; j.in_elem = in_elem; j.in_vec = 1;
                 j.out = task.output; j.out_elem = task.output_stride; j.out_vec = 1;
                 j.vectors = vectors;
                 j.conv = conv;
-                groups[{1, 2, v->half_bandwidth, in_kind, task.sample}].push_back(it);
+                it.plan = r.v;
+                groups[{1, on_ring ? 10 : 2, v->half_bandwidth, in_kind, task.sample, on_ring ? r.v->ring_window : 0}]
+                    .push_back(it);
             } else {
                 auto &j = it.axis;
                 j.plan = r.v->view;
@@ -1290,7 +1305,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
     launches.clear();
     for (auto &[key, items] : groups) {
         const bool fused = key.kind == 9;
-        const bool is_stream = (key.kind >= 2 && key.kind <= 6) || fused;
+        const bool is_stream = (key.kind >= 2 && key.kind <= 6) || fused || ring_kind(key.kind);
         const bool ring = ring_kind(key.kind);
         int per_block = key.kind == 2 ? stream_block : fused ? kScoreCtaThreads
                       : ring ? kTRingThreads : is_stream ? tstream_threads : kSeqThreads;
@@ -1307,7 +1322,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
         // Transposing kernels are assigned warps, not CTAs: a CTA's warps
         // may serve consecutive jobs of one plan (they share the CTA's record
         // copies), so only plan changes round up to a whole CTA.
-        const bool by_warp = (key.kind >= 3 && key.kind <= 6) || fused;
+        const bool by_warp = (key.kind >= 3 && key.kind <= 6) || fused || ring;
         const int warps_per_cta = per_block / 32;
         // Jobs of one plan stay together (they share record copies); plans
         // with the longest vectors come first, so that the CTAs that take
@@ -1322,18 +1337,26 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
         int per_lane = 1;
         if (key.kind == 4) {
             per_lane = 2;
-        } else if (key.kind == 3) {
+        } else if (ring) {
             // The split does not depend on the vectors a lane: neither do the
             // results.
-            items = segment_items(items, 32, segment_mode, warp_slots);
+            items = key.kind == 3 ? segment_items(items, 32, segment_mode, warp_slots)
+                                  : segment_items(items, 32, segment_mode, warp_slots, kAxisMargin, kAxisMinChunks);
             long warps = 0;
             for (const auto &it : items) warps += (it.stream.vectors + 31) / 32;
             if (!vectors_per_warp && warps >= kPairingWarps * static_cast<long>(warp_slots / kTResidentWarps))
                 per_lane = 2;
         }
         if (ring)
-            for (auto &it : items)
-                map_input(it.stream, key.in, it.stream.plan.source_size, it.tile_vectors, per_lane);
+            for (auto &it : items) {
+                auto &j = it.stream;
+                if (key.kind == 10 && key.pass == 1) {
+                    map_input_columns(j, j.plan.source_size, per_lane);
+                } else {
+                    map_input(j, key.in, j.plan.source_size, it.tile_vectors, per_lane);
+                    if (key.kind == 10) map_output_rows(j, j.plan.destination_size, per_lane);
+                }
+            }
         int warps = 0;
         const float *run_plan = nullptr;
         int run_chunk = 0;
@@ -1412,7 +1435,10 @@ void Executor::Impl::launch(const Compiled &c, const char *device_table, cudaStr
                                l.hb, l.variant ? 8 : 0, l.in, l.out, l.record_floats, stream);
         } else if (ring_kind(l.kind)) {
             rc = launch_tring(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
-                              l.variant & 31, l.per_lane, (l.variant & kTiled) != 0, l.in, l.out, stream);
+                              l.variant & 31, l.per_lane,
+                              l.kind == 10 ? (l.pass ? RingLayout::columns : RingLayout::rows)
+                              : l.variant & kTiled ? RingLayout::tiled : RingLayout::plain,
+                              l.in, l.out, stream);
         } else if (l.kind == 2) {
             rc = launch_stream(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks,
                                l.hb, kStreamChunk, l.pass == 0, l.in, l.out, l.record_floats,
@@ -2217,7 +2243,12 @@ std::unique_ptr<PreparedBatch> Executor::prepare_batch(const std::vector<PlaneTa
     // runs beside the other's first) for batches of many tasks that own
     // their scratch; split where the source pixels are halved.
     int n_parts = parts;
-    if (n_parts == 0) n_parts = !scratch && tasks.size() >= kSplitBatchTasks ? 2 : 1;
+    if (n_parts == 0) {
+        // One-axis passes have no second pass to run beside the first.
+        const auto planes = std::count_if(tasks.begin(), tasks.end(),
+                                          [](const PlaneTask &t) { return t.horizontal && t.vertical; });
+        n_parts = !scratch && static_cast<std::size_t>(planes) >= kSplitBatchTasks ? 2 : 1;
+    }
     if (n_parts != 1 && n_parts != 2) throw std::invalid_argument("a prepared batch has 1 or 2 parts");
     if (n_parts == 2 && (scratch || tasks.size() < 2))
         throw std::invalid_argument("two batch parts need two tasks and batch-owned scratch");

@@ -32,9 +32,12 @@ struct StreamPlanView {
 struct StreamJob {
     // Kernels with the ring in tensor memory: the tensor map of the input, used
     // when `mapped`: 1 a plane of contiguous vectors, 2 the intermediate in
-    // tiles of 32 samples.
+    // tiles of 32 samples, 3 a plane whose vectors are its columns.  One-axis
+    // rows: the output's, used when `out_mapped`.
     alignas(64) unsigned char map[128];
+    alignas(64) unsigned char out_map[128];
     std::int32_t mapped;
+    std::int32_t out_mapped;
     StreamPlanView plan;
     const void *in;
     std::int64_t in_elem, in_vec;
@@ -94,9 +97,12 @@ constexpr int kRingColumns = 48;
 constexpr int kTRingPitch = 34;
 // `chunk` is 32 or 64; contiguous = the vector's samples are adjacent
 // (rows: f32/u8/u16 in, f32 out); otherwise columns (f32 in; f32/u8/u16 out).
-// Transposing 2D passes, chunk-delayed, the sample ring in tensor memory
-// (tring_impl.cuh): vectors with adjacent samples in, destination-major output
-// with the vectors adjacent, or (`tiled`, Float32) in tiles of 32 vectors.
+// What a pass with the ring in tensor memory (tring_impl.cuh) reads and
+// writes: vectors with adjacent samples in and destination-major output with
+// the vectors adjacent, that output (Float32) in tiles of 32 vectors, a
+// Float32 plane's rows in and out, or its columns.
+enum class RingLayout : std::int32_t { plain, tiled, rows, columns };
+// Chunk-delayed passes, the sample ring in tensor memory (tring_impl.cuh).
 // Every job of a launch has the same window (StreamPack::ring_window) and its
 // plan view the matching records; `per_lane` vectors a lane (1 or 2), CTAs of kTRingThreads threads.
 constexpr int kTStreamThreads = 128;   // default CTA size of the two-pass kernels
@@ -104,7 +110,7 @@ constexpr int kTRingThreads = 128;
 constexpr int kTResidentWarps = 16;    // resident warps per SM (128 registers a thread)
 constexpr int kMinSegmentChunks = 1;   // shortest segment, in chunks (StreamJob)
 int launch_tring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
-                 int per_lane, bool tiled, dev::Sample in, dev::Sample out, void *stream);
+                 int per_lane, RingLayout layout, dev::Sample in, dev::Sample out, void *stream);
 
 // Columns passes with fused candidate scoring (tscore_impl.cuh): as
 // the transposing passes, for Float32 intermediates with chunk-delayed records

@@ -14,4 +14,11 @@ namespace dsmvc_gb {
 // aligned) keep mapped = 0.
 void map_input(dev::StreamJob &job, dev::Sample sample, int size, int tile_vectors, int per_lane);
 
+// One-axis passes over a Float32 plane: `job.map` of columns of `size`
+// samples, `job.in_elem` apart, boxes of 32 samples of 32 * `per_lane`
+// columns; `job.out_map` of rows of `size` samples, `job.out_vec` apart, boxes
+// of 32 samples of 32 * `per_lane` rows.
+void map_input_columns(dev::StreamJob &job, int size, int per_lane);
+void map_output_rows(dev::StreamJob &job, int size, int per_lane);
+
 } // namespace dsmvc_gb

@@ -25,6 +25,12 @@
 //  * Intermediate: in tiles of 32 rows, [row / 32][destination][row mod 32]:
 //    the first pass stores at constant offsets, the second reads 128
 //    contiguous bytes of each vector.
+//  * One-axis passes (RingLayout rows, columns): a row's 32 results of a chunk
+//    go to shared memory in the output map's swizzle and out by TMA, a
+//    column's samples come in boxes of 32 rows.  Their gather keeps the
+//    reference CUDA order.  Measured on one GB300, eight 1080p Float32 planes
+//    (one thread a vector, uncoalesced stores, before): rows to 1440 508 ->
+//    49 us, columns to 810 lines 381 -> 47 us.
 //  * Records: copied (cp.async) a chunk of 32 destinations at a time, three
 //    deep, for the CTA's four warps.  A warp-wide load of the same 16 bytes
 //    takes two shared-memory cycles, which is what two vectors a lane save.
@@ -96,17 +102,19 @@ template <class T> __device__ __forceinline__ T rout(float v, const Conversion &
 
 // ---- ring feeder ---------------------------------------------------------------
 
-template <class In, int V, int W>
+// LAYOUT columns: a vector's samples are a plane's column.
+template <class In, int V, int W, RingLayout LAYOUT>
 struct RingFeeder {
+    static constexpr bool COLS = LAYOUT == RingLayout::columns;
     static constexpr int SPL = 16 / static_cast<int>(sizeof(In));   // samples per 16 bytes
-    static constexpr int SB = 8 * SPL;                              // samples per staged block
+    static constexpr int SB = COLS ? 32 : 8 * SPL;                  // samples per staged block
     static constexpr int DUP = W <= 8 ? 8 : 16;                     // columns stored again after the ring
     static constexpr int VC = kRingColumns + 16;                    // columns per vector
     static constexpr int BUFFER = 32 * V * 128;                     // bytes per staging buffer
     static constexpr int NR = kRingStep * static_cast<int>(sizeof(In)) / 4;   // words of a step's samples
 
     const void *in;          // the plane
-    std::int64_t in_vec;
+    std::int64_t in_vec, in_elem;
     std::uint64_t map;       // its tensor map, 0: vectors not 16-byte aligned
     int first;               // the warp's first vector
     int vectors;             // its valid vectors (>= 1)
@@ -135,8 +143,8 @@ struct RingFeeder {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" :: "r"(mb), "r"(BUFFER) : "memory");
             asm volatile("cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes"
                          " [%0], [%1, {%2, %3, %4}], [%5];\n"
-                         :: "r"(stage + slot * BUFFER), "l"(map), "r"(tiled ? 0 : next), "r"(first),
-                            "r"(tiled ? next / 32 : 0), "r"(mb) : "memory");
+                         :: "r"(stage + slot * BUFFER), "l"(map), "r"(COLS ? first : tiled ? 0 : next),
+                            "r"(COLS ? next : first), "r"(tiled ? next / 32 : 0), "r"(mb) : "memory");
         }
         next += SB;
     }
@@ -181,6 +189,16 @@ struct RingFeeder {
     __device__ __forceinline__ void fetch(unsigned (&raw)[V][NR]) {
         if (map) {
             if (have % SB == 0) enter();
+            if constexpr (COLS) {
+                // [sample][column]: one load a sample.
+#pragma unroll
+                for (int a = 0; a < V; ++a)
+#pragma unroll
+                    for (int i = 0; i < NR; ++i)
+                        asm volatile("ld.shared.u32 %0, [%1];"
+                                     : "=r"(raw[a][i]) : "r"(at + row[a] + (have % SB + i) * (128 * V)));
+                return;
+            }
             // 16-byte pieces lie in the tensor map's 128-byte swizzle.
             const unsigned piece = (have % SB) / SPL;
 #pragma unroll
@@ -200,7 +218,8 @@ struct RingFeeder {
                 const In *p = static_cast<const In *>(in) + (first + min(lane + 32 * a, vectors - 1)) * in_vec;
                 In vals[kRingStep];
 #pragma unroll
-                for (int i = 0; i < kRingStep; ++i) vals[i] = __ldg(p + min(have + i, size - 1));
+                for (int i = 0; i < kRingStep; ++i)
+                    vals[i] = __ldg(p + (COLS ? min(have + i, size - 1) * in_elem : min(have + i, size - 1)));
 #pragma unroll
                 for (int i = 0; i < NR; ++i) {
                     unsigned w = 0;
@@ -310,7 +329,9 @@ template <int N> __device__ __forceinline__ void rload(float (&c)[N], const floa
 // Forward substitution of a chunk: its values to tensor memory at `ycol`
 // (column = destination of the chunk, a lane's vectors 64 columns apart).
 // `hist`: the HB values before it, oldest first.
-template <int HB, int W, int V, class Feed>
+// SPLIT: the gather's even and odd taps in two sums, else one after another
+// (the reference CUDA order, which one-axis passes keep).
+template <int HB, int W, int V, bool SPLIT, class Feed>
 __device__ __forceinline__ void rforward(float (&hist)[V][HB], const float *fwd, unsigned ycol, Feed &feed) {
     using R = RingRecord<HB, W>;
     constexpr int G = kRingGroup<V>;
@@ -342,7 +363,6 @@ __device__ __forceinline__ void rforward(float (&hist)[V][HB], const float *fwd,
 #pragma unroll
                     for (int a = 0; a < V; ++a) tm_ld<W>(x[(q + 1) & 1][a], at[(q + 1) & 3] + a * Feed::VC);
                 }
-                // Even and odd taps in the two halves, then their sum.
                 float2 acc[V];
 #pragma unroll
                 for (int a = 0; a < V; ++a) acc[a] = make_float2(0.0f, 0.0f);
@@ -352,13 +372,18 @@ __device__ __forceinline__ void rforward(float (&hist)[V][HB], const float *fwd,
 #pragma unroll
                     for (int a = 0; a < V; ++a) {
                         const float *xa = x[q & 1][a] + i;
-                        acc[a] = __ffma2_rn(make_float2(w.x, w.y), make_float2(xa[0], xa[1]), acc[a]);
-                        acc[a] = __ffma2_rn(make_float2(w.z, w.w), make_float2(xa[2], xa[3]), acc[a]);
+                        if constexpr (SPLIT) {
+                            acc[a] = __ffma2_rn(make_float2(w.x, w.y), make_float2(xa[0], xa[1]), acc[a]);
+                            acc[a] = __ffma2_rn(make_float2(w.z, w.w), make_float2(xa[2], xa[3]), acc[a]);
+                        } else {
+                            acc[a].x = fmaf(w.y, xa[1], fmaf(w.x, xa[0], acc[a].x));
+                            acc[a].x = fmaf(w.w, xa[3], fmaf(w.z, xa[2], acc[a].x));
+                        }
                     }
                 }
 #pragma unroll
                 for (int a = 0; a < V; ++a) {
-                    float sum = acc[a].x + acc[a].y;
+                    float sum = SPLIT ? acc[a].x + acc[a].y : acc[a].x;
 #pragma unroll
                     for (int e = 0; e < HB; ++e) sum = fmaf(lw[q * HB + e], y[a][t + q + e], sum);
                     // Records past the end of the vector are zero (inverse
@@ -383,11 +408,12 @@ __device__ __forceinline__ void rforward(float (&hist)[V][HB], const float *fwd,
 // on return).  MODE 0: the warm-up, nothing stored; 1: every result stored as
 // soon as it is known; 2: those of the chunk's first `valid` destinations.
 // `at`: the chunk's first destination; STEP: the output's destination stride,
-// 0: `out_elem`.
+// 0: `out_elem`, -1: rows, whose 32 results of a chunk go to `tile` in shared
+// memory (a row of 128 bytes each, in the output map's swizzle).
 template <int HB, int W, int V, int MODE, int STEP, class Out>
 __device__ __forceinline__ void rbackward(float (&carry)[V][HB], const float *bwd, unsigned ycol, int valid,
                                           Out *const (&out)[V], std::int64_t at, std::int64_t out_elem,
-                                          const Conversion &conv) {
+                                          const Conversion &conv, float *tile = nullptr) {
     using R = RingRecord<HB, W>;
     constexpr int G = kRingGroup<V>;
 #pragma unroll 1
@@ -402,7 +428,7 @@ __device__ __forceinline__ void rbackward(float (&carry)[V][HB], const float *bw
 #pragma unroll
             for (int d = 0; d < HB; ++d) x[a][G + d] = carry[a][d];
         Out *o[V];
-        if constexpr (MODE > 0) {
+        if constexpr (MODE > 0 && STEP >= 0) {
 #pragma unroll
             for (int a = 0; a < V; ++a) o[a] = out[a] + (STEP ? (at + tg) * STEP : (at + tg + G - 1) * out_elem);
         }
@@ -421,12 +447,21 @@ __device__ __forceinline__ void rbackward(float (&carry)[V][HB], const float *bw
                 for (int pos = 0; pos < HB; ++pos)
                     sum = fmaf(u[(t / 4) & 1][(t % 4) * HB + pos], x[a][t + (HB == 3 ? pos + 1 : HB - pos)], sum);
                 x[a][t] = y[a][t] - sum;
-                if constexpr (MODE > 0) {
+                if constexpr (MODE > 0 && STEP >= 0) {
                     Out *to = STEP ? o[a] + t * STEP : o[a];
                     if (MODE == 1 || tg + t < valid) *to = rout<Out>(x[a][t], conv);
                     if constexpr (STEP == 0) o[a] -= out_elem;
                 }
             }
+        }
+        if constexpr (MODE > 0 && STEP < 0) {
+            const int lane = threadIdx.x & 31;
+#pragma unroll
+            for (int a = 0; a < V; ++a)
+#pragma unroll
+                for (int t = 0; t < G; t += 4)
+                    *reinterpret_cast<float4 *>(tile + (32 * a + lane) * 32 + (((tg + t) / 4) ^ (lane & 7)) * 4) =
+                        make_float4(x[a][t], x[a][t + 1], x[a][t + 2], x[a][t + 3]);
         }
 #pragma unroll
         for (int a = 0; a < V; ++a)
@@ -435,21 +470,54 @@ __device__ __forceinline__ void rbackward(float (&carry)[V][HB], const float *bw
     }
 }
 
-// TILED: the output is the intermediate in tiles of 32 vectors,
-// [vector / 32][destination][vector mod 32].
-template <int HB, int W, int V, bool TILED, class In, class Out>
+// Writes a chunk's rows from `tile`: through the output's tensor map, which
+// clips what lies past the plane, or row by row.
+template <int V>
+__device__ __forceinline__ void rstore_rows(float *tile, std::uint64_t map, float *out, std::int64_t out_vec, int first,
+                                            int vectors, int at, int valid) {
+    const int lane = threadIdx.x & 31;
+    if (map) {
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+            asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];\n"
+                         :: "l"(map), "r"(at), "r"(first), "r"(0),
+                            "r"(static_cast<unsigned>(__cvta_generic_to_shared(tile))) : "memory");
+            asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+        }
+    } else {
+        __syncwarp();
+        for (int r = 0; r < vectors; ++r) {
+            const float v = tile[r * 32 + ((lane / 4) ^ (r & 7)) * 4 + lane % 4];
+            if (lane < valid) out[(first + r) * out_vec + at + lane] = v;
+        }
+        __syncwarp();
+    }
+}
+
+// The rows written so far have left `tile`.
+__device__ __forceinline__ void rstore_wait() {
+    if ((threadIdx.x & 31) == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+    __syncwarp();
+}
+
+template <int HB, int W, int V, RingLayout LAYOUT, class In, class Out>
 __global__ void __launch_bounds__(kRingThreads, 4 / V)
 tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
     using R = RingRecord<HB, W>;
-    using Feed = RingFeeder<In, V, W>;
-    constexpr int LC = kTChunk, WARPS = kRingThreads / 32, STEP = TILED ? 32 : 0;
+    using Feed = RingFeeder<In, V, W, LAYOUT>;
+    constexpr bool TILED = LAYOUT == RingLayout::tiled, ROWS = LAYOUT == RingLayout::rows;
+    constexpr bool SPLIT = LAYOUT == RingLayout::plain || TILED;
+    constexpr int LC = kTChunk, WARPS = kRingThreads / 32, STEP = TILED ? 32 : ROWS ? -1 : 0;
     constexpr int COLUMNS = 128 * V;       // the rings and two chunks of forward values
     static_assert(V * (Feed::VC + 2 * LC) <= COLUMNS);
     // Staging buffers (WARPS * kRingBuffers of Feed::BUFFER bytes, where the
-    // 128-byte swizzle's pattern of 1024 begins), then three chunks of records.
+    // 128-byte swizzle's pattern of 1024 begins), the rows of a chunk alike,
+    // then three chunks of records.
     extern __shared__ unsigned char ring_dynamic[];
     unsigned char *const ring_smem = ring_dynamic + (-static_cast<unsigned>(__cvta_generic_to_shared(ring_dynamic)) & 1023);
-    float *bufs = reinterpret_cast<float *>(ring_smem + WARPS * kRingBuffers * Feed::BUFFER);
+    unsigned char *const ring_rows = ring_smem + WARPS * kRingBuffers * Feed::BUFFER;
+    float *bufs = reinterpret_cast<float *>(ring_rows + (ROWS ? WARPS * V * 4096 : 0));
     __shared__ unsigned long long feed_bar[WARPS][kRingBuffers];
     __shared__ unsigned tm_base;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -463,12 +531,12 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
     const int n = p.destination_size;
     const int chunks = (n + LC - 1) / LC;
     // Chunks whose outputs this CTA stores: [ca, cb).  The forward
-    // substitution runs over [c0, ce]: from one chunk early (zero history)
-    // for a range past chunk 0, to one chunk late (the backward warm-up of
+    // substitution runs over [c0, ce]: from `margin` chunks early (zero
+    // history) for a range past chunk 0, to one chunk late (the backward warm-up of
     // the last stored chunk) for a range ending before the last chunk.
     const int ca = lead.chunk_begin;
     const int cb = lead.chunk_end > 0 ? lead.chunk_end : chunks;
-    const int c0 = ca > 0 ? ca - 1 : 0;
+    const int c0 = max(ca - lead.margin, 0);
     const int ce = cb < chunks ? cb : chunks - 1;
 
     tstage(bufs + (c0 % 3) * R::CHUNK, p, c0, tid, kRingThreads);
@@ -502,6 +570,7 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
     Feed feed;
     feed.in = job.in;
     feed.in_vec = job.in_vec;
+    feed.in_elem = job.in_elem;
     feed.map = job.mapped ? reinterpret_cast<std::uint64_t>(job.map) : 0;
     feed.first = idle ? 0 : warp_first;
     feed.vectors = idle ? 1 : left > 32 * V ? 32 * V : left;
@@ -515,7 +584,7 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
 #pragma unroll
     for (int a = 0; a < V; ++a) {
         const unsigned v = min(lane + 32 * a, feed.vectors - 1);
-        feed.row[a] = v * 128 + (v & 7) * 16;
+        feed.row[a] = Feed::COLS ? v * 4 : v * 128 + (v & 7) * 16;
     }
     feed.in_offset = job.conv.in_offset;
     feed.in_scale = job.conv.in_scale;
@@ -535,6 +604,16 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
 
     const Conversion conv = job.conv;
     const std::int64_t out_elem = job.out_elem;
+    float *const tile = reinterpret_cast<float *>(ring_rows + warp * V * 4096);
+    const std::uint64_t out_map = ROWS && job.out_mapped ? reinterpret_cast<std::uint64_t>(job.out_map) : 0;
+    if (out_map && lane == 0)
+        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" :: "l"(out_map) : "memory");
+    // A chunk's rows, once its last results are in `tile`.
+    auto rows = [&](int chunk) {
+        if constexpr (ROWS)
+            rstore_rows<V>(tile, out_map, static_cast<float *>(job.out), job.out_vec, feed.first, feed.vectors, chunk * LC,
+                           n - chunk * LC);
+    };
     const unsigned ycol = feed.ring + V * Feed::VC;        // chunk c's forward values 32 (c & 1) columns on
     float hist[V][HB], carry[V][HB];
 #pragma unroll
@@ -548,7 +627,7 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
         float *prev = bufs + ((c + 2) % 3) * R::CHUNK;
         if (!idle) {
             const unsigned yc = ycol + (c & 1) * LC, yp = ycol + (~c & 1) * LC;
-            rforward<HB, W, V>(hist, cur, yc, feed);
+            rforward<HB, W, V, SPLIT>(hist, cur, yc, feed);
             const float *cur_b = cur + R::GROUPS * R::GROUP;
 #pragma unroll
             for (int a = 0; a < V; ++a)
@@ -557,12 +636,19 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
             if (c + 1 == chunks) {
                 // The vector's last chunk: exact from the end, stored when the
                 // chunk is the CTA's.
-                rbackward<HB, W, V, 2, STEP>(carry, cur_b, yc, c < cb ? n - c * LC : 0, out, c * LC, out_elem, conv);
+                if constexpr (ROWS) rstore_wait();
+                rbackward<HB, W, V, 2, STEP>(carry, cur_b, yc, c < cb ? n - c * LC : 0, out, c * LC, out_elem, conv,
+                                             tile);
+                if (c < cb) rows(c);
             } else if (c > ca) {
                 rbackward<HB, W, V, 0, STEP>(carry, cur_b, yc, 0, out, 0, out_elem, conv);
             }
-            if (c > ca)
-                rbackward<HB, W, V, 1, STEP>(carry, prev + R::GROUPS * R::GROUP, yp, LC, out, (c - 1) * LC, out_elem, conv);
+            if (c > ca) {
+                if constexpr (ROWS) rstore_wait();
+                rbackward<HB, W, V, 1, STEP>(carry, prev + R::GROUPS * R::GROUP, yp, LC, out, (c - 1) * LC, out_elem, conv,
+                                             tile);
+                rows(c - 1);
+            }
         }
         if (c == ce) break;
         // Every warp is done with chunk c-1's records: fetch chunk c+2.
@@ -573,6 +659,9 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
     // No copy is left in flight; a stalled feed wait reports.
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     if (!idle) feed.drain();
+    if constexpr (ROWS) {
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
+    }
     if (__any_sync(0xffffffffu, feed.failed) && lane == 0) atomicOr(lead.status, dev::kStatusFeedStall);
     asm volatile("tcgen05.fence::before_thread_sync;\n");
     __syncthreads();
@@ -581,11 +670,12 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" :: "r"(tm), "n"(COLUMNS));
 }
 
-template <int HB, int W, int V, bool TILED, class In, class Out>
+template <int HB, int W, int V, RingLayout LAYOUT, class In, class Out>
 int rlaunch_typed(const StreamJob *jobs, int count, int blocks, cudaStream_t s) {
     constexpr int smem = 1024 + 3 * RingRecord<HB, W>::CHUNK * 4
-        + kRingThreads / 32 * kRingBuffers * RingFeeder<In, V, W>::BUFFER;
-    auto kernel = tring_kernel<HB, W, V, TILED, In, Out>;
+        + kRingThreads / 32 * (kRingBuffers * RingFeeder<In, V, W, LAYOUT>::BUFFER
+                               + (LAYOUT == RingLayout::rows ? V * 4096 : 0));
+    auto kernel = tring_kernel<HB, W, V, LAYOUT, In, Out>;
     static SmemLimit limit;
     if (const cudaError_t e = limit.ensure(kernel, smem); e != cudaSuccess) return static_cast<int>(e);
     kernel<<<blocks, kRingThreads, smem, s>>>(jobs, count);
@@ -593,25 +683,32 @@ int rlaunch_typed(const StreamJob *jobs, int count, int blocks, cudaStream_t s) 
 }
 
 template <int HB, int W, int V>
-int rlaunch(const StreamJob *jobs, int count, int blocks, dev::Sample in, dev::Sample out, bool tiled, void *stream) {
+int rlaunch(const StreamJob *jobs, int count, int blocks, dev::Sample in, dev::Sample out, RingLayout layout,
+            void *stream) {
     using dev::Sample;
     using std::uint16_t, std::uint8_t;
+    using L = RingLayout;
     const auto s = static_cast<cudaStream_t>(stream);
-    if (out == Sample::f32) {
-        if (in == Sample::f32)
-            return tiled ? rlaunch_typed<HB, W, V, true, float, float>(jobs, count, blocks, s)
-                         : rlaunch_typed<HB, W, V, false, float, float>(jobs, count, blocks, s);
-        if (in == Sample::u16)
-            return tiled ? rlaunch_typed<HB, W, V, true, uint16_t, float>(jobs, count, blocks, s)
-                         : rlaunch_typed<HB, W, V, false, uint16_t, float>(jobs, count, blocks, s);
-        if (in == Sample::u8)
-            return tiled ? rlaunch_typed<HB, W, V, true, uint8_t, float>(jobs, count, blocks, s)
-                         : rlaunch_typed<HB, W, V, false, uint8_t, float>(jobs, count, blocks, s);
+    if (in == Sample::f32 && out == Sample::f32) {
+        switch (layout) {
+        case L::plain: return rlaunch_typed<HB, W, V, L::plain, float, float>(jobs, count, blocks, s);
+        case L::tiled: return rlaunch_typed<HB, W, V, L::tiled, float, float>(jobs, count, blocks, s);
+        case L::rows: return rlaunch_typed<HB, W, V, L::rows, float, float>(jobs, count, blocks, s);
+        case L::columns: return rlaunch_typed<HB, W, V, L::columns, float, float>(jobs, count, blocks, s);
+        }
     }
-    if (in == Sample::f32 && out == Sample::u16)
-        return rlaunch_typed<HB, W, V, false, float, uint16_t>(jobs, count, blocks, s);
-    if (in == Sample::f32 && out == Sample::u8)
-        return rlaunch_typed<HB, W, V, false, float, uint8_t>(jobs, count, blocks, s);
+    if (out == Sample::f32 && layout == L::tiled) {
+        if (in == Sample::u16) return rlaunch_typed<HB, W, V, L::tiled, uint16_t, float>(jobs, count, blocks, s);
+        if (in == Sample::u8) return rlaunch_typed<HB, W, V, L::tiled, uint8_t, float>(jobs, count, blocks, s);
+    }
+    if (out == Sample::f32 && layout == L::plain) {
+        if (in == Sample::u16) return rlaunch_typed<HB, W, V, L::plain, uint16_t, float>(jobs, count, blocks, s);
+        if (in == Sample::u8) return rlaunch_typed<HB, W, V, L::plain, uint8_t, float>(jobs, count, blocks, s);
+    }
+    if (in == Sample::f32 && layout == L::plain) {
+        if (out == Sample::u16) return rlaunch_typed<HB, W, V, L::plain, float, uint16_t>(jobs, count, blocks, s);
+        if (out == Sample::u8) return rlaunch_typed<HB, W, V, L::plain, float, uint8_t>(jobs, count, blocks, s);
+    }
     return static_cast<int>(cudaErrorInvalidValue);
 }
 
