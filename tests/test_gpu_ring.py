@@ -46,6 +46,22 @@ def test_edges(gb, executor, whole_executor, paired_executor, kernel, taps, rati
                 assert err.max() <= INT_MAX_CODES, (sample, err.max())
 
 
+# Half-bandwidths 9 and 11 too, and a ratio beyond the ring's group refill.
+@pytest.mark.parametrize("width,height", SIZES)
+@pytest.mark.parametrize("kernel,taps,ratio", PLANS + [("spline64", 3, 1.5), ("lanczos", 5, 1.3), ("lanczos", 6, 1.2),
+                                                       ("bilinear", 3, 7.3)])
+def test_two_pass_edges(gb, exact_executor, kernel, taps, ratio, width, height):
+    """Two-pass kernels (xring_impl.cuh) in whole vectors: the reference CUDA
+    order bit for bit."""
+    h, v, oh, ov = pair(gb, kernel, taps, ratio, width, height)
+    for sample in ("f32", "u16", "u8"):
+        bits = {"f32": 16, "u16": 16, "u8": 8}[sample]
+        conv = gb.integer_conversion(bits, False, False) if sample != "f32" else None
+        x = make_input(height, width, sample, 4)
+        want = O.inverse_2d_gpu_order(oh, ov, x, conv) if conv else O.inverse_2d_gpu_order(oh, ov, x)
+        assert np.array_equal(exact_executor.inverse_2d(h, v, x, conv), want), sample
+
+
 @pytest.mark.parametrize("sample", ["f32", "u16", "u8"])
 def test_unaligned_and_paired_batches(gb, whole_executor, sample):
     """Planes whose rows no tensor map admits (an odd pitch) and a batch large

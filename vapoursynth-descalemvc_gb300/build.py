@@ -31,9 +31,10 @@ HOST_SOURCES = ["planner.cpp", "stream_plan.cpp", "executor.cpp", "sweep.cpp", "
                 "host_blocks.cpp", "tensor_map.cpp", "capi.cpp"]
 TRING_SOURCES = [f"tring_hb{hb}_w{w}.cu" for hb, ws in ((1, (4, 8, 16)), (3, (8, 12, 16)), (5, (8, 12, 16)),
                                                       (7, (12, 16))) for w in ws]
+XRING_SOURCES = [f"x{s[1:]}" for s in TRING_SOURCES] + ["xring_hb9_w16.cu", "xring_hb11_w16.cu"]
 TSOLVE_SOURCES = ([f"tsolve_hb{hb}.cu" for hb in (1, 3, 5, 7, 9, 11)]
                   + [f"tsolve64_hb{hb}.cu" for hb in (1, 3, 5, 7, 9, 11)])
-CUDA_SOURCES = TRING_SOURCES + TSOLVE_SOURCES + ["kernels.cu", "stream.cu", "stream_hb1.cu", "stream_hb3.cu",
+CUDA_SOURCES = TRING_SOURCES + XRING_SOURCES + TSOLVE_SOURCES + ["kernels.cu", "stream.cu", "stream_hb1.cu", "stream_hb3.cu",
                 "stream_hb5.cu", "stream_hb7.cu", "tscore_hb1.cu", "tscore_hb3.cu", "tscore_hb5.cu",
                 "tscore_hb7.cu", "noalloc.cu", "score.cu", "peak.cu", "gpu_planner.cu", "refine64.cu"]
 

@@ -98,7 +98,6 @@ struct DevicePlan {
     bool stream_u16 = false, stream_u8 = false;
     bool stream_t = false;          // transposing 2D kernels admitted
     bool stream_x = false;          // two-pass transposing 2D kernels admitted
-    bool stream_xg = false;         // ... with the grouped refill of window 8
     bool stream64 = false;          // Float64 two-pass transposing kernels admitted
     bool stream64_seg = false;      // ... and their segments (StreamPack64::segmentable)
     int margin64 = 0;
@@ -217,7 +216,6 @@ void finish_plan(DevicePlan *dp, const AxisPlan &p, const PlanImage &img, char *
         dp->exact_margin = pack.exact_margin;
         if (dp->stream_seg || dp->exact_margin) dp->chunk_first_block = pack.chunk_first_block;
         dp->stream_x = pack.exact;
-        dp->stream_xg = pack.exact && pack.ring_ok_transposed && pack.window == 8;
         auto &sv = dp->stream_view;
         sv.source_size = p.source_size;
         sv.destination_size = p.destination_size;
@@ -736,13 +734,9 @@ bool stream_row_ok(const DevicePlan &dp, dev::Sample in) {
 // intermediate.
 constexpr int kTiled = 32;
 
-// Launch-group variant of a transposing pass.  Chunk-delayed kernels (3, 4):
-// their window.  Two-pass kernels: 1 runs the window-8 kernels with the
-// grouped refill.
-int compiled_window(const DevicePlan &dp, int kind) {
-    if (kind == 5) return dp.stream_xg ? 1 : 0;
-    return dp.ring_window;
-}
+// Launch-group variant of a Float32 transposing pass: its compiled window; 0
+// on the two-pass kernels with the ring in shared memory.
+int compiled_window(const DevicePlan &dp) { return dp.ring_window; }
 
 // Launches of at least this many warps an SM (at one vector a lane) run two
 // vectors a lane: a record's load then serves both, and four warps an SM stay.
@@ -943,7 +937,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
             r.transposed = true;
             auto pass_kind = [&](const DevicePlan &dp) {
                 if (!allow_stream) return 0;
-                const bool delayed = dp.stream && dp.ring_window;
+                const bool delayed = dp.stream_t && dp.ring_window;
                 if (dp.stream_x && (prefer_exact || !delayed)) return 5;
                 if (delayed) return vectors_per_warp == 64 ? 4 : 3;
                 return 0;
@@ -956,9 +950,11 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                     throw std::invalid_argument("fused scoring needs a chunk-delayed Float32 columns pass");
                 r.v_kind = 9;
             }
-            // Between two chunk-delayed passes the intermediate is tiled,
+            // Between two passes with the ring in tensor memory the
+            // intermediate is tiled,
             // [row / 32][destination][row mod 32].
-            r.tiled = ring_kind(r.h_kind) && ring_kind(r.v_kind) && v->source_size >= 32;
+            auto on_ring = [](const DevicePlan &dp, int kind) { return ring_kind(kind) || (kind == 5 && dp.ring_window); };
+            r.tiled = on_ring(*r.h, r.h_kind) && on_ring(*r.v, r.v_kind) && v->source_size >= 32;
             const std::size_t whole = r.tiled ? 32 : 4;
             r.mid_stride = (static_cast<std::size_t>(v->source_size) + whole - 1) / whole * whole;
             r.mid = bytes;
@@ -1146,7 +1142,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                 * sample_bytes(task.sample);
             if (r.h_kind) {
                 auto &j = hi.stream;
-                j.plan = r.h_kind == 5 ? r.h->stream_view : r.h->ring_view;
+                j.plan = r.h->ring_window ? r.h->ring_view : r.h->stream_view;
                 j.in = task.input; j.in_elem = 1; j.in_vec = task.input_stride;
                 j.out = mid; j.out_elem = pitch; j.out_vec = 1;
                 j.y = mid; j.y_elem = pitch;                // forward values in place
@@ -1154,9 +1150,9 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                 j.conv = conv;
                 hi.plan = r.h;
                 auto &group = groups[{0, r.h_kind, h->half_bandwidth, task.sample, dev::Sample::f32,
-                                      compiled_window(*r.h, r.h_kind) | (r.tiled ? kTiled : 0)}];
+                                      compiled_window(*r.h) | (r.tiled ? kTiled : 0)}];
                 if (r.h_kind == 5)
-                    push_segments(group, hi, r.h->chunk_first_block, r.h->exact_margin, h->destination_size, r.seg_h,
+                    push_segments(group, hi, r.h->ring_window ? r.h->ring_first_block : r.h->chunk_first_block, r.h->exact_margin, h->destination_size, r.seg_h,
                                   base + r.yseg_h, pitch, 4);
                 else
                     group.push_back(hi);
@@ -1183,7 +1179,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                 groups[{1, 9, v->half_bandwidth, dev::Sample::f32, dev::Sample::f32, fused_window(*r.v)}].push_back(vi);
             } else if (r.v_kind) {
                 auto &j = vi.stream;
-                j.plan = r.v_kind == 5 ? r.v->stream_view : r.v->ring_view;
+                j.plan = r.v->ring_window ? r.v->ring_view : r.v->stream_view;
                 j.in = mid; j.in_elem = 1; j.in_vec = r.tiled ? 32 : pitch;
                 vi.tile_vectors = r.tiled ? h->destination_size : 0;
                 j.out = task.output; j.out_elem = task.output_stride; j.out_vec = 1;
@@ -1198,9 +1194,9 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                 j.conv = conv;
                 vi.plan = r.v;
                 auto &group = groups[{1, r.v_kind, v->half_bandwidth, dev::Sample::f32, task.sample,
-                                      compiled_window(*r.v, r.v_kind)}];
+                                      compiled_window(*r.v)}];
                 if (r.v_kind == 5)
-                    push_segments(group, vi, r.v->chunk_first_block, r.v->exact_margin, v->destination_size, r.seg_v,
+                    push_segments(group, vi, r.v->ring_window ? r.v->ring_first_block : r.v->chunk_first_block, r.v->exact_margin, v->destination_size, r.seg_v,
                                   base + r.yseg_v, static_cast<std::int64_t>(h->destination_size), 4);
                 else
                     group.push_back(vi);
@@ -1234,7 +1230,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
             if (!v) it.bytes += static_cast<std::uint64_t>(vectors) * h->destination_size * 4;
             if (r.h_stream) {
                 auto &j = it.stream;
-                const bool on_ring = !v && r.h->ring_window;
+                const bool on_ring = !v && r.h->stream_t && r.h->ring_window;
                 j.plan = on_ring ? r.h->ring_view : r.h->stream_view;
                 j.in = in; j.in_elem = 1; j.in_vec = in_vec;
                 j.out = out; j.out_elem = 1; j.out_vec = out_vec;
@@ -1270,7 +1266,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
             if (!h) it.bytes += static_cast<std::uint64_t>(vectors) * v->source_size * 4;
             if (r.v_stream) {
                 auto &j = it.stream;
-                const bool on_ring = !h && r.v->ring_window;
+                const bool on_ring = !h && r.v->stream_t && r.v->ring_window;
                 j.plan = on_ring ? r.v->ring_view : r.v->stream_view;
                 j.in = in; j.in_elem = in_elem; j.in_vec = 1;
                 j.out = task.output; j.out_elem = task.output_stride; j.out_vec = 1;
@@ -1306,7 +1302,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
     for (auto &[key, items] : groups) {
         const bool fused = key.kind == 9;
         const bool is_stream = (key.kind >= 2 && key.kind <= 6) || fused || ring_kind(key.kind);
-        const bool ring = ring_kind(key.kind);
+        const bool ring = ring_kind(key.kind) || (key.kind == 5 && key.variant);
         int per_block = key.kind == 2 ? stream_block : fused ? kScoreCtaThreads
                       : ring ? kTRingThreads : is_stream ? tstream_threads : kSeqThreads;
         if (tuning && key.kind != 2 && !ring && key.kind <= 6) {
@@ -1340,8 +1336,9 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
         } else if (ring) {
             // The split does not depend on the vectors a lane: neither do the
             // results.
-            items = key.kind == 3 ? segment_items(items, 32, segment_mode, warp_slots)
-                                  : segment_items(items, 32, segment_mode, warp_slots, kAxisMargin, kAxisMinChunks);
+            if (key.kind == 3) items = segment_items(items, 32, segment_mode, warp_slots);
+            if (key.kind == 10)
+                items = segment_items(items, 32, segment_mode, warp_slots, kAxisMargin, kAxisMinChunks);
             long warps = 0;
             for (const auto &it : items) warps += (it.stream.vectors + 31) / 32;
             if (!vectors_per_warp && warps >= kPairingWarps * static_cast<long>(warp_slots / kTResidentWarps))
@@ -1431,8 +1428,11 @@ void Executor::Impl::launch(const Compiled &c, const char *device_table, cudaStr
             rc = launch_tsolve64(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.threads,
                                  l.hb, l.in, l.out, l.record_floats, f64_fused, status, stream);
         } else if (l.kind == 5) {
-            rc = launch_tsolve(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.threads,
-                               l.hb, l.variant ? 8 : 0, l.in, l.out, l.record_floats, stream);
+            rc = l.variant & 31
+                ? launch_xring(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
+                               l.variant & 31, l.per_lane, (l.variant & kTiled) != 0, l.in, l.out, stream)
+                : launch_tsolve(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.threads,
+                                l.hb, l.in, l.out, l.record_floats, stream);
         } else if (ring_kind(l.kind)) {
             rc = launch_tring(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
                               l.variant & 31, l.per_lane,

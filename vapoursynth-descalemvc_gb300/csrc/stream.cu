@@ -33,12 +33,12 @@ int launch_stream(const dev::StreamJob *jobs, int job_count, int total_blocks, i
 
 namespace dsmvc_gb {
 
-int launch_tsolve_hb1(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tsolve_hb3(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tsolve_hb5(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tsolve_hb7(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tsolve_hb9(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
-int launch_tsolve_hb11(const dev::StreamJob *, int, int, int, int, dev::Sample, dev::Sample, int, void *);
+int launch_tsolve_hb1(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
+int launch_tsolve_hb3(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
+int launch_tsolve_hb5(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
+int launch_tsolve_hb7(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
+int launch_tsolve_hb9(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
+int launch_tsolve_hb11(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, void *);
 
 int launch_tsolve64_hb1(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, bool, std::uint32_t *, void *);
 int launch_tsolve64_hb3(const dev::StreamJob *, int, int, int, dev::Sample, dev::Sample, int, bool, std::uint32_t *, void *);
@@ -66,14 +66,14 @@ bool tsolve_supports(int half_bandwidth) {
 }
 
 int launch_tsolve(const dev::StreamJob *jobs, int job_count, int total_blocks, int threads, int half_bandwidth,
-                  int window, dev::Sample in, dev::Sample out, int record_floats, void *stream) {
+                  dev::Sample in, dev::Sample out, int record_floats, void *stream) {
     switch (half_bandwidth) {
-    case 1: return launch_tsolve_hb1(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-    case 3: return launch_tsolve_hb3(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-    case 5: return launch_tsolve_hb5(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-    case 7: return launch_tsolve_hb7(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-    case 9: return launch_tsolve_hb9(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
-    case 11: return launch_tsolve_hb11(jobs, job_count, total_blocks, threads, window, in, out, record_floats, stream);
+    case 1: return launch_tsolve_hb1(jobs, job_count, total_blocks, threads, in, out, record_floats, stream);
+    case 3: return launch_tsolve_hb3(jobs, job_count, total_blocks, threads, in, out, record_floats, stream);
+    case 5: return launch_tsolve_hb5(jobs, job_count, total_blocks, threads, in, out, record_floats, stream);
+    case 7: return launch_tsolve_hb7(jobs, job_count, total_blocks, threads, in, out, record_floats, stream);
+    case 9: return launch_tsolve_hb9(jobs, job_count, total_blocks, threads, in, out, record_floats, stream);
+    case 11: return launch_tsolve_hb11(jobs, job_count, total_blocks, threads, in, out, record_floats, stream);
     default: return static_cast<int>(cudaErrorInvalidValue);
     }
 }
@@ -114,6 +114,51 @@ int launch_tring(const dev::StreamJob *jobs, int job_count, int total_blocks, in
         return launch_tring_hb7_w12(jobs, job_count, total_blocks, per_lane, layout, in, out, stream);
     if (half_bandwidth == 7 && window == 16)
         return launch_tring_hb7_w16(jobs, job_count, total_blocks, per_lane, layout, in, out, stream);
+    return static_cast<int>(cudaErrorInvalidValue);
+}
+
+int launch_xring_hb1_w4(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb1_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb1_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb3_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb3_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb3_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb5_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb5_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb5_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb7_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb7_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb9_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+int launch_xring_hb11_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, void *);
+
+int launch_xring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
+                 int per_lane, bool tiled, dev::Sample in, dev::Sample out, void *stream) {
+    if (half_bandwidth == 1 && window == 4)
+        return launch_xring_hb1_w4(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 1 && window == 8)
+        return launch_xring_hb1_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 1 && window == 16)
+        return launch_xring_hb1_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 3 && window == 8)
+        return launch_xring_hb3_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 3 && window == 12)
+        return launch_xring_hb3_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 3 && window == 16)
+        return launch_xring_hb3_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 5 && window == 8)
+        return launch_xring_hb5_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 5 && window == 12)
+        return launch_xring_hb5_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 5 && window == 16)
+        return launch_xring_hb5_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 7 && window == 12)
+        return launch_xring_hb7_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 7 && window == 16)
+        return launch_xring_hb7_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 9 && window == 16)
+        return launch_xring_hb9_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
+    if (half_bandwidth == 11 && window == 16)
+        return launch_xring_hb11_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, stream);
     return static_cast<int>(cudaErrorInvalidValue);
 }
 

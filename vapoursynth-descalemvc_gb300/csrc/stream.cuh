@@ -120,12 +120,16 @@ int launch_tring(const dev::StreamJob *jobs, int job_count, int total_blocks, in
 int launch_tscore(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
                   int record_floats, void *stream);
 
-// Two-pass transposing 2D passes (tsolve_impl.cuh): exact forward and
-// backward sweeps through the jobs' forward-value planes; half-bandwidths
-// 1..11 (odd).
+// Two-pass transposing 2D passes: exact forward and backward sweeps through
+// the jobs' forward-value planes; half-bandwidths 1..11 (odd).  launch_xring
+// (xring_impl.cuh, the ring in tensor memory) takes the windows and records
+// of launch_tring; launch_tsolve (tsolve_impl.cuh) serves the plans whose
+// group refill exceeds that ring.
+int launch_xring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
+                 int per_lane, bool tiled, dev::Sample in, dev::Sample out, void *stream);
 bool tsolve_supports(int half_bandwidth);
 int launch_tsolve(const dev::StreamJob *jobs, int job_count, int total_blocks, int threads, int half_bandwidth,
-                  int window, dev::Sample in, dev::Sample out, int record_floats, void *stream);
+                  dev::Sample in, dev::Sample out, int record_floats, void *stream);
 
 // Float64 two-pass transposing 2D passes (tsolve64_impl.cuh) for plans that
 // retain Float64: the first pass reads u8/u16/f32 and writes the Float64

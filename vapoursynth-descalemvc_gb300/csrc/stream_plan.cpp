@@ -48,6 +48,7 @@ bool ring_fits_grouped(const std::vector<int> &s0, int window, int size, int rin
 int ring_window(int half_bandwidth, int window) {
     // Half-bandwidth 1 windows are 4 samples below a ratio of 1.5; wider
     // kernels' never are.
+    if (half_bandwidth > 7) return window <= 16 ? 16 : 0;
     if (half_bandwidth == 1 && window <= 4) return 4;
     if (half_bandwidth <= 5 && window <= 8) return 8;
     if (half_bandwidth >= 3 && window <= 12) return 12;
@@ -284,7 +285,7 @@ StreamPack pack_stream_plan(const AxisPlan &p, int chunk, int ring, bool hb_supp
     out.chunk_first_block.resize(static_cast<std::size_t>(chunks));
     for (int k = 0; k < chunks; ++k) out.chunk_first_block[static_cast<std::size_t>(k)] = s0[static_cast<std::size_t>(k) * chunk] / 16 * 16;
 
-    const int rw = delayed && out.ring_ok_transposed ? ring_window(hb, window) : 0;
+    const int rw = (delayed && out.ring_ok_transposed) || out.exact ? ring_window(hb, window) : 0;
     if (rw) {
         // Replay of the refills: sixteen samples at a time, up to the end of
         // the group's last window.  (A source shorter than the compiled

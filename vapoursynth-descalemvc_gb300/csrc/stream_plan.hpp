@@ -62,7 +62,8 @@ struct StreamPack {
     std::vector<float> forward;     // * forward_stride
     std::vector<float> backward;    // * backward_stride
     // Records of the 2D kernels with the ring in tensor memory
-    // (tring_impl.cuh), when the plan is eligible and their feed fits: the
+    // (tring_impl.cuh, xring_impl.cuh), when the plan is eligible or exact and
+    // their feed fits: the
     // window is ring_window(hb, window) samples, starting at most at
     // source_size - ring_window.  Per group of four destinations: their four
     // ring columns (start mod kRingColumns), the first word also holding the refill

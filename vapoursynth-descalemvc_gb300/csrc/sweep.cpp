@@ -593,8 +593,8 @@ struct Sweep::Impl {
         for (const int threads : {64, 128, 256}) {
             BatchTuning all;
             for (const auto &g : keys) {
-                // The chunk-delayed kernels have one CTA size.
-                const bool ring = g.kind == 3 || g.kind == 4;
+                // The kernels with the ring in tensor memory have one CTA size.
+                const bool ring = g.kind == 3 || g.kind == 4 || (g.kind == 5 && g.key[5]);
                 const int most = g.kind >= 3 && !ring ? 256 : 128;
                 if (g.kind != 2 && g.kind <= 6 && threads <= most && (!ring || threads == 128)) all[g.key] = threads;
             }

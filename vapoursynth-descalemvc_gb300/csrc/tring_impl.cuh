@@ -134,6 +134,36 @@ struct RingFeeder {
     bool tiled;
     bool failed;             // a wait ran out: nothing more is fetched or waited for
 
+    // `stage_at`, `mbar_at`: the warp's staging buffers and their barriers.
+    __device__ __forceinline__ void init(const StreamJob &j, int samples, int first_vector, int count_vectors, int l,
+                                         unsigned ring_at, unsigned stage_at, unsigned mbar_at) {
+        in = j.in;
+        in_vec = j.in_vec;
+        in_elem = j.in_elem;
+        map = j.mapped ? reinterpret_cast<std::uint64_t>(j.map) : 0;
+        first = first_vector;
+        vectors = count_vectors;
+        size = limit = samples;
+        lane = l;
+        ring = ring_at;
+        stage = stage_at;
+        mbar = mbar_at;
+        // Lanes past the warp's last vector repeat it: same samples, same
+        // results, stored to the same place.
+#pragma unroll
+        for (int a = 0; a < V; ++a) {
+            const unsigned v = min(lane + 32 * a, vectors - 1);
+            row[a] = COLS ? v * 4 : v * 128 + (v & 7) * 16;
+        }
+        in_offset = j.conv.in_offset;
+        in_scale = j.conv.in_scale;
+        tiled = j.mapped == 2;
+        failed = false;
+        if (map && lane == 0)
+            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" :: "l"(map) : "memory");
+        __syncwarp();
+    }
+
     // Fetches the block at `next` into buffer `slot`.
     __device__ __forceinline__ void issue(unsigned slot) {
         unsigned elected;
@@ -326,13 +356,13 @@ template <int N> __device__ __forceinline__ void rload(float (&c)[N], const floa
     }
 }
 
-// Forward substitution of a chunk: its values to tensor memory at `ycol`
-// (column = destination of the chunk, a lane's vectors 64 columns apart).
-// `hist`: the HB values before it, oldest first.
+// Forward substitution of a chunk: store(a, t, y) takes eight values of a
+// vector from destination t of the chunk on.  `hist`: the HB values before it,
+// oldest first.
 // SPLIT: the gather's even and odd taps in two sums, else one after another
 // (the reference CUDA order, which one-axis passes keep).
-template <int HB, int W, int V, bool SPLIT, class Feed>
-__device__ __forceinline__ void rforward(float (&hist)[V][HB], const float *fwd, unsigned ycol, Feed &feed) {
+template <int HB, int W, int V, bool SPLIT, class Feed, class Store>
+__device__ __forceinline__ void rforward(float (&hist)[V][HB], const float *fwd, Feed &feed, Store &&store) {
     using R = RingRecord<HB, W>;
     constexpr int G = kRingGroup<V>;
 #pragma unroll 1
@@ -395,12 +425,11 @@ __device__ __forceinline__ void rforward(float (&hist)[V][HB], const float *fwd,
 #pragma unroll
         for (int a = 0; a < V; ++a) {
 #pragma unroll
-            for (int t = 0; t < G; t += 8) tm_st8(ycol + a * 2 * kTChunk + tg + t, &y[a][HB + t]);
+            for (int t = 0; t < G; t += 8) store(a, tg + t, &y[a][HB + t]);
 #pragma unroll
             for (int d = 0; d < HB; ++d) hist[a][d] = y[a][G + d];
         }
     }
-    tm_wait_st();
 }
 
 // Backward substitution of a chunk from its forward values at `ycol` and the
@@ -568,31 +597,10 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
     const bool idle = left <= 0;
     const unsigned tm = tm_base;
     Feed feed;
-    feed.in = job.in;
-    feed.in_vec = job.in_vec;
-    feed.in_elem = job.in_elem;
-    feed.map = job.mapped ? reinterpret_cast<std::uint64_t>(job.map) : 0;
-    feed.first = idle ? 0 : warp_first;
-    feed.vectors = idle ? 1 : left > 32 * V ? 32 * V : left;
-    feed.size = feed.limit = p.source_size;
-    feed.lane = lane;
-    feed.ring = tm + (static_cast<unsigned>(warp * 32) << 16);
-    feed.stage = static_cast<unsigned>(__cvta_generic_to_shared(ring_smem + warp * kRingBuffers * Feed::BUFFER));
-    feed.mbar = static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][0]));
-    // Lanes past the warp's last vector repeat it: same samples, same results,
-    // stored to the same place.
-#pragma unroll
-    for (int a = 0; a < V; ++a) {
-        const unsigned v = min(lane + 32 * a, feed.vectors - 1);
-        feed.row[a] = Feed::COLS ? v * 4 : v * 128 + (v & 7) * 16;
-    }
-    feed.in_offset = job.conv.in_offset;
-    feed.in_scale = job.conv.in_scale;
-    feed.tiled = job.mapped == 2;
-    feed.failed = false;
-    if (feed.map && lane == 0)
-        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" :: "l"(feed.map) : "memory");
-    __syncwarp();
+    feed.init(job, p.source_size, idle ? 0 : warp_first, idle ? 1 : min(left, 32 * V), lane,
+              tm + (static_cast<unsigned>(warp * 32) << 16),
+              static_cast<unsigned>(__cvta_generic_to_shared(ring_smem + warp * kRingBuffers * Feed::BUFFER)),
+              static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][0])));
     if (!idle) feed.start(c0 > 0 ? lead.first_sample : 0);
 
     Out *out[V];
@@ -627,7 +635,8 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
         float *prev = bufs + ((c + 2) % 3) * R::CHUNK;
         if (!idle) {
             const unsigned yc = ycol + (c & 1) * LC, yp = ycol + (~c & 1) * LC;
-            rforward<HB, W, V, SPLIT>(hist, cur, yc, feed);
+            rforward<HB, W, V, SPLIT>(hist, cur, feed, [&](int a, int t, const float *y) { tm_st8(yc + a * 2 * LC + t, y); });
+            tm_wait_st();
             const float *cur_b = cur + R::GROUPS * R::GROUP;
 #pragma unroll
             for (int a = 0; a < V; ++a)

@@ -4,11 +4,9 @@
 
 namespace dsmvc_gb {
 
-int launch_tsolve_hb7(const dev::StreamJob *jobs, int count, int blocks, int threads, int window,
-                       dev::Sample in, dev::Sample out, int record_floats, void *stream) {
-    auto s = static_cast<cudaStream_t>(stream);
-    if (window == 8) return xlaunch_k<7, 8>(jobs, count, blocks, threads, in, out, record_floats, s);
-    return xlaunch_k<7, 0>(jobs, count, blocks, threads, in, out, record_floats, s);
+int launch_tsolve_hb7(const dev::StreamJob *jobs, int count, int blocks, int threads, dev::Sample in,
+                       dev::Sample out, int record_floats, void *stream) {
+    return xlaunch_hb<7>(jobs, count, blocks, threads, in, out, record_floats, static_cast<cudaStream_t>(stream));
 }
 
 } // namespace dsmvc_gb

@@ -15,8 +15,9 @@
 //
 // Nothing is approximated, so the results equal the reference CUDA kernels'
 // bit for bit, for any decay of the factors and half-bandwidths up to 11.
-// The ring is refilled per destination (windows up to 16 samples), or per
-// group of four destinations for window 8 where the host's replay admits it.
+// The ring is refilled per destination (windows up to 16 samples): these
+// kernels serve the plans whose refill per group of four destinations
+// exceeds the ring of xring_impl.cuh (ratios beyond about 5).
 // The forward plane is the output itself where it is a Float32 plane with
 // the output's layout (the first pass's intermediate, Float32 outputs), else
 // a caller scratch plane.  Registers hold one chunk at a time.
@@ -27,7 +28,7 @@
 namespace dsmvc_gb {
 namespace {
 
-template <int HB, int K, class In, class Out>
+template <int HB, class In, class Out>
 __global__ void __launch_bounds__(kTMaxThreads)
 tsolve_kernel(const StreamJob *__restrict__ jobs, int job_count, int record_floats) {
     constexpr int LC = kTChunk;
@@ -84,8 +85,8 @@ tsolve_kernel(const StreamJob *__restrict__ jobs, int job_count, int record_floa
     // region starts at its first computed destination).
     float *yplane = job.y + v - static_cast<std::int64_t>(ybase) * job.y_elem;
     Out *out = static_cast<Out *>(job.out) + v;
-    const int fs = fwd_stride<HB, K>(p), bs = bwd_stride<HB, K>(p);
-    const int kw = K > 0 ? K : p.window;
+    const int fs = fwd_stride<HB, 0>(p), bs = bwd_stride<HB, 0>(p);
+    const int kw = p.window;
 
     // ---- forward sweep ---------------------------------------------------
     tstage(bufs + (fc0 % 3) * per_buffer, p, fc0, tid, nthreads);
@@ -104,36 +105,17 @@ tsolve_kernel(const StreamJob *__restrict__ jobs, int job_count, int record_floa
             float y[LC];
 #pragma unroll
             for (int t = 0; t < LC; ++t) {
-                if constexpr (K > 0) {
-                    // Window 8: one refill per group of four destinations.
-                    if (t % 4 == 0) {
-                        const int s_last = __float_as_int(fwd[(t + 3) * fs]);
-                        const int need = max(s_last, __float_as_int(fwd[t * fs])) + kw;
-                        feed.ensure(min(need, p.source_size));
-                    }
-                }
                 const float *rec = fwd + t * fs;
                 const float4 hdr = tlds4(rec);
-                if constexpr (K == 0) feed.ensure(min(__float_as_int(hdr.x) + kw, p.source_size));
+                feed.ensure(min(__float_as_int(hdr.x) + kw, p.source_size));
                 const float *win = feed.ring + lane + __float_as_int(hdr.z);
                 float sum = 0.0f;
-                if constexpr (K > 0) {
-#pragma unroll
-                    for (int k = 0; k < K; k += 4) {
-                        const float4 w = tlds4(rec + 4 + k);
-                        sum = fmaf(w.x, win[(k + 0) * kTPitch], sum);
-                        sum = fmaf(w.y, win[(k + 1) * kTPitch], sum);
-                        sum = fmaf(w.z, win[(k + 2) * kTPitch], sum);
-                        sum = fmaf(w.w, win[(k + 3) * kTPitch], sum);
-                    }
-                } else {
-                    for (int k = 0; k < kw; k += 4) {
-                        const float4 w = tlds4(rec + 4 + k);
-                        sum = fmaf(w.x, win[(k + 0) * kTPitch], sum);
-                        sum = fmaf(w.y, win[(k + 1) * kTPitch], sum);
-                        sum = fmaf(w.z, win[(k + 2) * kTPitch], sum);
-                        sum = fmaf(w.w, win[(k + 3) * kTPitch], sum);
-                    }
+                for (int k = 0; k < kw; k += 4) {
+                    const float4 w = tlds4(rec + 4 + k);
+                    sum = fmaf(w.x, win[(k + 0) * kTPitch], sum);
+                    sum = fmaf(w.y, win[(k + 1) * kTPitch], sum);
+                    sum = fmaf(w.z, win[(k + 2) * kTPitch], sum);
+                    sum = fmaf(w.w, win[(k + 3) * kTPitch], sum);
                 }
                 const float *low = rec + 4 + kw;
 #pragma unroll
@@ -215,31 +197,31 @@ tsolve_kernel(const StreamJob *__restrict__ jobs, int job_count, int record_floa
     }
 }
 
-template <int HB, int K, class In, class Out>
+template <int HB, class In, class Out>
 int xlaunch_typed(const StreamJob *jobs, int count, int blocks, int threads, int record_floats, cudaStream_t s) {
     if (threads < 32 || threads > kTMaxThreads || threads % 32) return static_cast<int>(cudaErrorInvalidValue);
     const int smem = (3 * kTChunk * record_floats + threads / 32 * kTRingFloats) * static_cast<int>(sizeof(float));
-    auto kernel = tsolve_kernel<HB, K, In, Out>;
+    auto kernel = tsolve_kernel<HB, In, Out>;
     static SmemLimit limit;
     if (const cudaError_t e = limit.ensure(kernel, smem); e != cudaSuccess) return static_cast<int>(e);
     kernel<<<blocks, threads, smem, s>>>(jobs, count, record_floats);
     return static_cast<int>(cudaGetLastError());
 }
 
-template <int HB, int K>
-int xlaunch_k(const StreamJob *jobs, int count, int blocks, int threads, dev::Sample in, dev::Sample out,
+template <int HB>
+int xlaunch_hb(const StreamJob *jobs, int count, int blocks, int threads, dev::Sample in, dev::Sample out,
               int record_floats, cudaStream_t s) {
     using dev::Sample;
     if (in == Sample::f32 && out == Sample::f32)
-        return xlaunch_typed<HB, K, float, float>(jobs, count, blocks, threads, record_floats, s);
+        return xlaunch_typed<HB, float, float>(jobs, count, blocks, threads, record_floats, s);
     if (in == Sample::u16 && out == Sample::f32)
-        return xlaunch_typed<HB, K, std::uint16_t, float>(jobs, count, blocks, threads, record_floats, s);
+        return xlaunch_typed<HB, std::uint16_t, float>(jobs, count, blocks, threads, record_floats, s);
     if (in == Sample::u8 && out == Sample::f32)
-        return xlaunch_typed<HB, K, std::uint8_t, float>(jobs, count, blocks, threads, record_floats, s);
+        return xlaunch_typed<HB, std::uint8_t, float>(jobs, count, blocks, threads, record_floats, s);
     if (in == Sample::f32 && out == Sample::u16)
-        return xlaunch_typed<HB, K, float, std::uint16_t>(jobs, count, blocks, threads, record_floats, s);
+        return xlaunch_typed<HB, float, std::uint16_t>(jobs, count, blocks, threads, record_floats, s);
     if (in == Sample::f32 && out == Sample::u8)
-        return xlaunch_typed<HB, K, float, std::uint8_t>(jobs, count, blocks, threads, record_floats, s);
+        return xlaunch_typed<HB, float, std::uint8_t>(jobs, count, blocks, threads, record_floats, s);
     return static_cast<int>(cudaErrorInvalidValue);
 }
 

@@ -1,0 +1,13 @@
+// Two-pass transposing kernels with the ring in tensor memory,
+// half-bandwidth 5, windows of 12 samples.
+#include "xring_impl.cuh"
+
+namespace dsmvc_gb {
+
+int launch_xring_hb5_w12(const dev::StreamJob *jobs, int count, int blocks, int per_lane, bool tiled,
+                       dev::Sample in, dev::Sample out, void *stream) {
+    return per_lane == 2 ? xrlaunch<5, 12, 2>(jobs, count, blocks, in, out, tiled, stream)
+                         : xrlaunch<5, 12, 1>(jobs, count, blocks, in, out, tiled, stream);
+}
+
+} // namespace dsmvc_gb
