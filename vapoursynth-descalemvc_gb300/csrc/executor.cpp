@@ -571,6 +571,7 @@ struct Executor::Impl {
     // Default CTA size of the transposing kernels (DSMVC_GB_TSTREAM_THREADS,
     // 32..256 in multiples of 32); batches may tune it per launch group.
     int tstream_threads = kTStreamThreads;
+    int tsolve64_threads = kTSolve64Threads;
     // Segments of the chunk-delayed transposing passes (DSMVC_GB_SEGMENTS):
     // 0 automatic (a launch group whose warps leave the GPU's resident warp
     // slots unfilled splits its vectors into up to slots / warps ranges of
@@ -1304,7 +1305,8 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
         const bool is_stream = (key.kind >= 2 && key.kind <= 6) || fused || ring_kind(key.kind);
         const bool ring = ring_kind(key.kind) || (key.kind == 5 && key.variant);
         int per_block = key.kind == 2 ? stream_block : fused ? kScoreCtaThreads
-                      : ring ? kTRingThreads : is_stream ? tstream_threads : kSeqThreads;
+                      : ring ? kTRingThreads : key.kind == 6 ? tsolve64_threads : is_stream ? tstream_threads
+                      : kSeqThreads;
         if (tuning && key.kind != 2 && !ring && key.kind <= 6) {
             const GroupTuple g{key.pass, key.kind, key.hb, static_cast<int>(key.in), static_cast<int>(key.out),
                                key.variant};
@@ -1598,7 +1600,7 @@ Executor::Executor(int device) : impl_(std::make_unique<Impl>()) {
     if (const char *env = std::getenv("DSMVC_GB_TSTREAM_THREADS")) {
         char *end = nullptr;
         const long v = std::strtol(env, &end, 10);
-        if (end && *end == '\0' && v >= 32 && v <= 256 && v % 32 == 0) impl_->tstream_threads = static_cast<int>(v);
+        if (end && *end == '\0' && v >= 32 && v <= 256 && v % 32 == 0) impl_->tstream_threads = impl_->tsolve64_threads = static_cast<int>(v);
     }
     if (const char *env = std::getenv("DSMVC_GB_SEGMENTS")) {
         char *end = nullptr;

@@ -106,6 +106,11 @@ enum class RingLayout : std::int32_t { plain, tiled, rows, columns };
 // Every job of a launch has the same window (StreamPack::ring_window) and its
 // plan view the matching records; `per_lane` vectors a lane (1 or 2), CTAs of kTRingThreads threads.
 constexpr int kTStreamThreads = 128;   // default CTA size of the two-pass kernels
+// Float64 two-pass kernels: two warps a CTA spread a launch's segments more
+// evenly over the SMs, whose FP64 units bind (4K Spline64 frames on one
+// GB300, 128 threads against 64: one 1826 and 1661 us, four 3468 and 3369,
+// sixteen 9514 and 9433).
+constexpr int kTSolve64Threads = 64;
 constexpr int kTRingThreads = 128;
 constexpr int kTResidentWarps = 16;    // resident warps per SM (128 registers a thread)
 constexpr int kMinSegmentChunks = 1;   // shortest segment, in chunks (StreamJob)
