@@ -6,10 +6,11 @@
 // whose transpose the plan stores as a CSR by destination.  Upscaling a
 // descaled plane Y (rows x cols) back to the source size is A_v * Y * A_h^T.
 // One kernel computes, per column tile and segment of source rows, the row
-// pass Z = Y * A_h^T for the descaled rows the segment needs (in shared
-// memory), then A_v * Z, |. - frame| and one partial sum per block of 16
-// rows.  Partial sums are reduced in a fixed order, so a score does not
-// depend on launch shapes or on the other candidates of the sweep.
+// pass Z = Y * A_h^T for the descaled rows the segment needs, then A_v * Z,
+// |. - frame| and partial sums per block of 16 rows.  Partial sums are reduced
+// in a fixed order, so a score does not depend on launch shapes or on the
+// other candidates of the sweep.  Two forms: operators whose windows are short
+// and move forward (score_walk_kernel), and any others (score_tiles_kernel).
 #pragma once
 
 #include <cstdint>
@@ -32,7 +33,9 @@ struct ScoreJob {
     std::int64_t frame_stride;
     std::int32_t width, height;
     ForwardCsr h, v;                // forward operators of the two axes
-    float *partials;                // row blocks x column tiles
+    float *partials;                // `parts` sums
+    std::int32_t parts;
+    std::int32_t taps;              // dense windows of score_walk_kernel (2, 4, 6 or 8), 0: score_tiles_kernel
     float *score;                   // the candidate's score
     std::int32_t first_block;       // scoring blocks before this job
     std::int32_t segment_rows;      // source rows per scoring block (a multiple of kScoreRowBlock)
@@ -86,6 +89,13 @@ constexpr int kScoreMaxSegmentRows = 256;    // rows of a segment whose entry ra
 // (their row-pass values are staged in shared memory).
 int launch_score_tiles(const dev::ScoreJob *jobs, int job_count, int total_blocks, int max_span_rows,
                        void *stream);
+// The same for jobs with `taps`: a block of kScoreWalkThreads threads per
+// (column tile, row segment of at most kScoreWalkRows rows).
+constexpr int kScoreWalkThreads = kScoreThreads / 2;   // two columns a thread
+constexpr int kScoreWalkRows = 128;
+constexpr int kScoreWalkAhead = 8;                     // rows staged ahead
+constexpr int kScoreWalkSpan = 96;                     // descaled columns under 64 source columns
+int launch_score_walk(const dev::ScoreJob *jobs, int job_count, int total_blocks, void *stream);
 // *jobs[i].score = sum of job i's partials / (width * height), one block
 // per job, in a fixed order.
 int launch_score_finalize(const dev::ScoreJob *jobs, int job_count, void *stream);

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <bit>
 #include <array>
 #include <chrono>
 #include <climits>
@@ -52,6 +53,48 @@ struct HostForward {
     std::vector<std::int32_t> indices;
     std::vector<float> weights;
 };
+
+// The dense windows with which score_walk_kernel can read an operator, bit k
+// for 2 k + 2 samples (k < 4).  Vertically: every row's entries within the
+// window from min(first, descaled - window) on, those starts never decreasing.
+// Horizontally: at most the window's entries a column, those of every two
+// columns 2u, 2u + 1 within one sample more, and those of a warp's 64 columns
+// within its staging.
+unsigned walk_windows(const HostForward &f, int descaled, bool vertical) {
+    const int rows = static_cast<int>(f.offsets.size()) - 1;
+    auto count = [&](int r) { return static_cast<int>(f.offsets[static_cast<std::size_t>(r) + 1] - f.offsets[static_cast<std::size_t>(r)]); };
+    auto first = [&](int r) { return f.indices[f.offsets[static_cast<std::size_t>(r)]]; };
+    auto last = [&](int r) { return f.indices[f.offsets[static_cast<std::size_t>(r) + 1] - 1]; };
+    int most = 0;
+    for (int r = 0; r < rows; ++r) {
+        if (count(r) == 0) return 0;
+        most = std::max(most, count(r));
+    }
+    unsigned out = 0;
+    for (int k = 0; k < 4; ++k) {
+        const int taps = 2 * k + 2, span = vertical ? taps : taps + 1;
+        bool ok = descaled >= span && most <= taps;
+        int previous = 0;
+        for (int r = 0; r < rows && ok; r += vertical ? 1 : 2) {
+            const bool two = !vertical && r + 1 < rows;
+            const int start = std::min(two ? std::min(first(r), first(r + 1)) : first(r), descaled - span);
+            const int end = two ? std::max(last(r), last(r + 1)) : last(r);
+            ok = end - start < span && (!vertical || start >= previous);
+            previous = start;
+        }
+        for (int r = 0; r < rows && ok && !vertical; r += 64) {
+            int low = INT32_MAX, high = 0;
+            for (int q = r; q < std::min(rows, r + 64); ++q) {
+                const int start = std::min(first(q), descaled - span);
+                low = std::min(low, start);
+                high = std::max(high, start + span);
+            }
+            ok = high - low <= kScoreWalkSpan;
+        }
+        if (ok) out |= 1U << k;
+    }
+    return out;
+}
 
 HostForward forward_csr(const AxisPlan &p) {
     HostForward f;
@@ -138,7 +181,8 @@ struct Sweep::Impl {
         int column_blocks = 0;
         std::array<int, 4> max_span{};   // per entry of kSegments (unfused candidates)
         int fused_first = 0, fused = 0;       // its fused candidates' epilogues
-        int unfused_first = 0, unfused = 0;   // its unfused candidates' score jobs
+        int unfused_first = 0, unfused = 0;   // its unfused candidates' score jobs,
+        int walk = 0, walk_blocks = 0;        // those of score_walk_kernel first
     };
     std::vector<Wave> waves;
     std::vector<std::size_t> y_offset, partial_offset;   // within a wave's buffers
@@ -157,6 +201,7 @@ struct Sweep::Impl {
     std::size_t scratch_capacity = 0;
     std::map<const AxisPlan *, dev::ForwardCsr> forward;
     std::map<const AxisPlan *, HostForward> host_forward;   // while building
+    std::map<const AxisPlan *, std::array<unsigned, 2>> windows;   // walk_windows: horizontal, vertical
     int segment_rows = 32;
     int best_segment = 32;
     int vectors_per_warp = 0;   // 0: the executor's default; 32 / 64 once tuned
@@ -198,6 +243,7 @@ struct Sweep::Impl {
             c.indices = reinterpret_cast<const std::int32_t *>(put(f.indices.data(), f.indices.size() * 4));
             c.weights = reinterpret_cast<const float *>(put(f.weights.data(), f.weights.size() * 4));
             forward[p] = c;
+            windows[p] = {walk_windows(f, p->destination_size, false), walk_windows(f, p->destination_size, true)};
             std::array<int, 4> sp{};
             for (std::size_t k = 0; k < sp.size(); ++k) {
                 const int seg = kSegments[k];
@@ -405,7 +451,8 @@ struct Sweep::Impl {
     // and partial sums.
     void plan_waves() {
         const std::size_t budget = options.memory_budget ? options.memory_budget : (32ULL << 30);
-        const std::size_t partials = align_up(static_cast<std::size_t>(column_tiles()) * segments(kScoreRowBlock) * 4);
+        const std::size_t partials = align_up(static_cast<std::size_t>(column_tiles()) * segments(kScoreRowBlock) * 4
+                                              * (kScoreWalkThreads / 32));
         std::size_t y_bytes = 0, p_bytes = 0, s_bytes = 0;
         std::size_t y_max = 0, p_max = 0, s_max = 0;
         y_offset.assign(candidates.size(), 0);
@@ -469,6 +516,17 @@ struct Sweep::Impl {
         scratch_mem.allocate(s_max);
         scratch_capacity = s_max;
         for (auto &w : waves) {
+            int at = w.unfused_first;
+            for (const bool walk : {true, false}) {
+                for (int k = 0; k < w.count; ++k) {
+                    const std::size_t i = static_cast<std::size_t>(w.first + k);
+                    if (unfused_of[i] < 0 || (walk_window(i) > 0) != walk) continue;
+                    unfused_of[i] = at++;
+                    w.walk += walk ? 1 : 0;
+                }
+            }
+        }
+        for (auto &w : waves) {
             for (int k = 0; k < w.count; ++k) {
                 const std::size_t i = static_cast<std::size_t>(w.first + k);
                 PlaneTask t = task_of(i);
@@ -478,16 +536,31 @@ struct Sweep::Impl {
         }
     }
 
-    // Score jobs of the unfused candidates (in candidate order) with `seg`
-    // source rows per column-pass block; block numbering restarts at each
-    // wave (`plain`: at each job).
+    // The candidate's window in score_walk_kernel, 0 where it needs the other.
+    [[nodiscard]] int walk_window(std::size_t i) const {
+        const unsigned both = windows.at(candidates[i].first)[0] & windows.at(candidates[i].second)[1];
+        return both ? 2 * std::countr_zero(both) + 2 : 0;
+    }
+
+    // Score jobs of the unfused candidates (per wave, those of
+    // score_walk_kernel first) with `seg` source rows per block; block
+    // numbering restarts at each wave's two launches (`plain`: at each job).
     std::vector<dev::ScoreJob> score_jobs(int seg, bool plain) {
         std::vector<dev::ScoreJob> jobs(static_cast<std::size_t>(unfused_count));
         for (auto &w : waves) {
             int cols = 0;
+            w.walk_blocks = 0;
+            std::vector<std::size_t> order(static_cast<std::size_t>(w.unfused));
             for (int k = 0; k < w.count; ++k) {
                 const std::size_t i = static_cast<std::size_t>(w.first + k);
-                if (unfused_of[i] < 0) continue;
+                if (unfused_of[i] >= 0) order[static_cast<std::size_t>(unfused_of[i] - w.unfused_first)] = i;
+            }
+            for (std::size_t q = 0; q < order.size(); ++q) {
+                const std::size_t i = order[q];
+                if (static_cast<int>(q) == w.walk) {
+                    w.walk_blocks = cols;
+                    cols = 0;
+                }
                 const AxisPlan *h = candidates[i].first, *v = candidates[i].second;
                 auto &j = jobs[static_cast<std::size_t>(unfused_of[i])];
                 j.descaled = reinterpret_cast<const float *>(y_mem.data() + y_offset[i]);
@@ -505,7 +578,13 @@ struct Sweep::Impl {
                 j.segment_rows = seg;
                 j.column_tiles = column_tiles();
                 j.first_block = plain ? 0 : cols;
+                j.taps = walk_window(i);
+                j.parts = j.column_tiles * segments(kScoreRowBlock) * (j.taps ? kScoreWalkThreads / 32 : 1);
                 cols += j.column_tiles * segments(seg);
+            }
+            if (w.walk == w.unfused) {
+                w.walk_blocks = cols;
+                cols = 0;
             }
             w.column_blocks = cols;
         }
@@ -530,11 +609,18 @@ struct Sweep::Impl {
         return 0;
     }
 
+    // The re-upscale and error sums of a wave's unfused candidates.
+    void enqueue_errors(const Wave &w, cudaStream_t s) {
+        check(launch_score_walk(wave_jobs(w), w.walk, w.walk_blocks, s), "launching scoring");
+        check(launch_score_tiles(wave_jobs(w) + w.walk, w.unfused - w.walk, w.column_blocks, span_rows(w), s),
+              "launching scoring");
+    }
+
     // A wave's scores are reduced before the next wave reuses its buffers
     // (descaled planes and partial sums).
     void enqueue_scoring(const Wave &w, cudaStream_t s) {
         if (w.unfused) {
-            check(launch_score_tiles(wave_jobs(w), w.unfused, w.column_blocks, span_rows(w), s), "launching scoring");
+            enqueue_errors(w, s);
             check(launch_score_finalize(wave_jobs(w), w.unfused, s), "launching score finalize");
         }
         if (w.fused)
@@ -619,9 +705,7 @@ struct Sweep::Impl {
             if (w.max_span[k] > kMaxSpanRows) continue;
             upload_jobs(job_mem, score_jobs(kSegments[k], false));
             segment_rows = kSegments[k];
-            const float ms = time_ms([&] {
-                check(launch_score_tiles(wave_jobs(w), w.unfused, w.column_blocks, span_rows(w), stream), "launching");
-            }, 1);
+            const float ms = time_ms([&] { enqueue_errors(w, stream); }, 1);
             if (!any || ms < best_ms) {
                 best_ms = ms;
                 any = true;
@@ -727,7 +811,8 @@ void Sweep::run_plain(void *stream) {
                 for (std::size_t q = 0; q < std::size(kSegments); ++q)
                     if (kSegments[q] == m.segment_rows) span = m.spans.at(v)[q];
                 const dev::ScoreJob *job = jobs + m.unfused_of[i];
-                check(launch_score_tiles(job, 1, col_blocks, span, s), "launching");
+                check(m.walk_window(i) ? launch_score_walk(job, 1, col_blocks, s)
+                                       : launch_score_tiles(job, 1, col_blocks, span, s), "launching");
                 check(launch_score_finalize(job, 1, s), "launching");
             }
             check(cudaStreamSynchronize(s), "synchronizing");
@@ -746,8 +831,7 @@ std::array<double, 3> Sweep::stage_milliseconds(void *stream) {
             check(cudaEventRecord(ev[0], s), "recording event");
             w.batch->launch(s);
             check(cudaEventRecord(ev[1], s), "recording event");
-            if (w.unfused)
-                check(launch_score_tiles(m.wave_jobs(w), w.unfused, w.column_blocks, m.span_rows(w), s), "launching");
+            if (w.unfused) m.enqueue_errors(w, s);
             check(cudaEventRecord(ev[2], s), "recording event");
             if (w.unfused) check(launch_score_finalize(m.wave_jobs(w), w.unfused, s), "launching");
             if (w.fused) check(launch_fused_score_finalize(m.epilogues + w.fused_first, w.fused, s), "launching");
@@ -785,7 +869,8 @@ SweepInfo Sweep::info() const {
     i.device_bytes = m.forward_mem.bytes + m.y_mem.bytes + m.partial_mem.bytes + m.scratch_mem.bytes
         + m.job_mem.bytes + m.plain_job_mem.bytes + m.score_mem.bytes + m.epilogue_mem.bytes;
     for (const auto &w : m.waves)
-        i.kernel_launches += w.batch->kernel_launches() + (w.unfused ? 2 : 0) + (w.fused ? 1 : 0);
+        i.kernel_launches += w.batch->kernel_launches() + (w.walk ? 1 : 0) + (w.walk < w.unfused ? 1 : 0)
+            + (w.unfused ? 1 : 0) + (w.fused ? 1 : 0);
     i.fused_candidates = m.fused_count;
     i.tune_milliseconds = m.tune_ms;
     i.segment_rows = m.segment_rows;
