@@ -51,6 +51,11 @@ constexpr int kSeqThreads = 128;   // threads per block of the sequential kernel
 // Prepared batches of at least this many 2D tasks (and their own scratch) run
 // as two parts on two streams.
 constexpr std::size_t kSplitBatchTasks = 8;
+// Prepared batches in one part with a pass of at least this many launches
+// (plans of different kernels) run them side by side: each alone leaves most
+// SMs idle (a 1080p sweep of 189 candidates, seven launches a pass: 2418 us one
+// after another, 1784 side by side).
+constexpr std::size_t kBranchLaunches = 3, kMaxBranches = 8;
 std::size_t align_up(std::size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
 
 std::size_t sample_bytes(dev::Sample s) {
@@ -695,6 +700,7 @@ struct Executor::Impl {
                  const std::function<char *(std::size_t)> &scratch, std::uint32_t *status,
                  const Tuning *tuning = nullptr, int vectors_per_warp = 0);
     void launch(const Compiled &c, const char *device_table, cudaStream_t stream, std::uint32_t *status);
+    void launch(const Launch &l, const char *device_table, cudaStream_t stream, std::uint32_t *status);
     // `copies`: a stream holding the tasks' input copies; the job table is
     // copied behind them there and the kernels wait for both.
     void enqueue(Workspace &ws, const std::vector<PlaneTask> &tasks, char *scratch = nullptr,
@@ -1399,62 +1405,64 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
     out.tasks = tasks.size();
 }
 
+void Executor::Impl::launch(const Launch &l, const char *device_table, cudaStream_t stream, std::uint32_t *status) {
+    Record *rec = nullptr;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(stream, &capturing);
+    if (profiling && capturing == cudaStreamCaptureStatusNone) {
+        std::scoped_lock lock(mutex);
+        records.emplace_back();
+        rec = &records.back();
+        rec->name = kernel_name({l.pass, l.kind, l.hb, l.in, l.out, l.variant});
+        rec->bytes = l.bytes;
+        rec->start = pooled_event();
+        rec->stop = pooled_event();
+        cuda_check(cudaEventRecord(rec->start, stream), "recording event");
+    }
+    const char *dev_table = device_table + l.offset;
+    int rc = 0;
+    if (l.kind == 9) {
+        rc = launch_tscore(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
+                           l.variant, l.record_floats, stream);
+    } else if (l.kind == 7) {
+        rc = launch_refine64(reinterpret_cast<const dev::AxisJob *>(dev_table), l.count, l.blocks, l.threads,
+                             l.hb, l.in, status, stream);
+    } else if (l.kind == 8) {
+        rc = launch_convert64(reinterpret_cast<const dev::AxisJob *>(dev_table), l.count, l.blocks, l.threads,
+                              l.out, status, stream);
+    } else if (l.kind == 6) {
+        rc = launch_tsolve64(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.threads,
+                             l.hb, l.in, l.out, l.record_floats, f64_fused, status, stream);
+    } else if (l.kind == 5) {
+        rc = l.variant & 31
+            ? launch_xring(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
+                           l.variant & 31, l.per_lane, (l.variant & kTiled) != 0, l.in, l.out, stream)
+            : launch_tsolve(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.threads,
+                            l.hb, l.in, l.out, l.record_floats, stream);
+    } else if (ring_kind(l.kind)) {
+        rc = launch_tring(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
+                          l.variant & 31, l.per_lane,
+                          l.kind == 10 ? (l.pass ? RingLayout::columns : RingLayout::rows)
+                          : l.variant & kTiled ? RingLayout::tiled : RingLayout::plain,
+                          l.in, l.out, stream);
+    } else if (l.kind == 2) {
+        rc = launch_stream(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks,
+                           l.hb, kStreamChunk, l.pass == 0, l.in, l.out, l.record_floats,
+                           stream);
+    } else if (l.kind == 1) {
+        rc = launch_axis_f64(reinterpret_cast<const dev::AxisJob *>(dev_table), l.count, l.blocks,
+                             l.threads, l.hb, l.in, l.out, status, stream);
+    } else {
+        rc = launch_axis_f32(reinterpret_cast<const dev::AxisJob *>(dev_table), l.count, l.blocks,
+                             l.threads, l.hb, l.in, l.out, stream);
+    }
+    cuda_check(rc, "launching axis kernel");
+    if (rec) cuda_check(cudaEventRecord(rec->stop, stream), "recording event");
+}
+
 void Executor::Impl::launch(const Compiled &c, const char *device_table, cudaStream_t stream,
                             std::uint32_t *status) {
-    for (const auto &l : c.launches) {
-        Record *rec = nullptr;
-        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-        cudaStreamIsCapturing(stream, &capturing);
-        if (profiling && capturing == cudaStreamCaptureStatusNone) {
-            std::scoped_lock lock(mutex);
-            records.emplace_back();
-            rec = &records.back();
-            rec->name = kernel_name({l.pass, l.kind, l.hb, l.in, l.out, l.variant});
-            rec->bytes = l.bytes;
-            rec->start = pooled_event();
-            rec->stop = pooled_event();
-            cuda_check(cudaEventRecord(rec->start, stream), "recording event");
-        }
-        const char *dev_table = device_table + l.offset;
-        int rc = 0;
-        if (l.kind == 9) {
-            rc = launch_tscore(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
-                               l.variant, l.record_floats, stream);
-        } else if (l.kind == 7) {
-            rc = launch_refine64(reinterpret_cast<const dev::AxisJob *>(dev_table), l.count, l.blocks, l.threads,
-                                 l.hb, l.in, status, stream);
-        } else if (l.kind == 8) {
-            rc = launch_convert64(reinterpret_cast<const dev::AxisJob *>(dev_table), l.count, l.blocks, l.threads,
-                                  l.out, status, stream);
-        } else if (l.kind == 6) {
-            rc = launch_tsolve64(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.threads,
-                                 l.hb, l.in, l.out, l.record_floats, f64_fused, status, stream);
-        } else if (l.kind == 5) {
-            rc = l.variant & 31
-                ? launch_xring(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
-                               l.variant & 31, l.per_lane, (l.variant & kTiled) != 0, l.in, l.out, stream)
-                : launch_tsolve(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.threads,
-                                l.hb, l.in, l.out, l.record_floats, stream);
-        } else if (ring_kind(l.kind)) {
-            rc = launch_tring(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
-                              l.variant & 31, l.per_lane,
-                              l.kind == 10 ? (l.pass ? RingLayout::columns : RingLayout::rows)
-                              : l.variant & kTiled ? RingLayout::tiled : RingLayout::plain,
-                              l.in, l.out, stream);
-        } else if (l.kind == 2) {
-            rc = launch_stream(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks,
-                               l.hb, kStreamChunk, l.pass == 0, l.in, l.out, l.record_floats,
-                               stream);
-        } else if (l.kind == 1) {
-            rc = launch_axis_f64(reinterpret_cast<const dev::AxisJob *>(dev_table), l.count, l.blocks,
-                                 l.threads, l.hb, l.in, l.out, status, stream);
-        } else {
-            rc = launch_axis_f32(reinterpret_cast<const dev::AxisJob *>(dev_table), l.count, l.blocks,
-                                 l.threads, l.hb, l.in, l.out, stream);
-        }
-        cuda_check(rc, "launching axis kernel");
-        if (rec) cuda_check(cudaEventRecord(rec->stop, stream), "recording event");
-    }
+    for (const auto &l : c.launches) launch(l, device_table, stream, status);
     std::scoped_lock lock(mutex);
     stats.launches += c.launches.size();
     stats.plane_tasks += c.tasks;
@@ -2083,6 +2091,22 @@ struct PreparedBatch::Impl {
     std::vector<std::unique_ptr<Part>> parts;
     cudaStream_t side = nullptr;           // the second part's stream
     cudaEvent_t fork = nullptr, join = nullptr;
+    // A batch in one part whose passes are many launches: the streams that
+    // run a pass's launches side by side, and their events.
+    struct Branch {
+        cudaStream_t stream = nullptr;
+        cudaEvent_t done = nullptr;
+        Branch() {
+            cuda_check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "creating stream");
+            cuda_check(cudaEventCreateWithFlags(&done, cudaEventDisableTiming), "creating event");
+        }
+        ~Branch() {
+            if (done) cudaEventDestroy(done);
+            if (stream) cudaStreamDestroy(stream);
+        }
+    };
+    std::vector<std::unique_ptr<Branch>> branches;
+    void launch_branches(cudaStream_t s);
     std::uint32_t *status = nullptr;       // device
     std::uint32_t *status_host = nullptr;  // pinned
     ~Impl() {
@@ -2112,10 +2136,41 @@ PreparedBatch::~PreparedBatch() {
     impl_.reset();
 }
 
+// A pass's launches on the caller's stream and the branches, forked from it and
+// joined back (capturable); those with the fewest, longest vectors (the later
+// kinds) first.
+void PreparedBatch::Impl::launch_branches(cudaStream_t s) {
+    const auto &launches = parts[0]->compiled.launches;
+    const char *table = parts[0]->table.data();
+    for (std::size_t first = 0; first < launches.size();) {
+        std::size_t end = first;
+        while (end < launches.size() && launches[end].pass == launches[first].pass) ++end;
+        const std::size_t used = std::min(branches.size(), end - first - 1);
+        if (used) cuda_check(cudaEventRecord(fork, s), "recording fork");
+        for (std::size_t k = 0; k < used; ++k) cuda_check(cudaStreamWaitEvent(branches[k]->stream, fork, 0), "forking");
+        for (std::size_t i = end, k = 0; i-- > first; ++k) {
+            const std::size_t b = k % (used + 1);
+            owner->launch(launches[i], table, b ? branches[b - 1]->stream : s, status);
+        }
+        for (std::size_t k = 0; k < used; ++k) {
+            cuda_check(cudaEventRecord(branches[k]->done, branches[k]->stream), "recording join");
+            cuda_check(cudaStreamWaitEvent(s, branches[k]->done, 0), "joining");
+        }
+        first = end;
+    }
+    std::scoped_lock lock(owner->mutex);
+    owner->stats.launches += launches.size();
+    owner->stats.plane_tasks += parts[0]->compiled.tasks;
+}
+
 void PreparedBatch::launch(void *stream) {
     DeviceGuard guard(impl_->owner->device);
     auto s = static_cast<cudaStream_t>(stream);
     auto &m = *impl_;
+    if (!m.branches.empty() && !m.owner->profiling) {
+        m.launch_branches(s);
+        return;
+    }
     if (m.parts.size() == 1) {
         m.owner->launch(m.parts[0]->compiled, m.parts[0]->table.data(), s, m.status);
         return;
@@ -2289,6 +2344,22 @@ std::unique_ptr<PreparedBatch> Executor::prepare_batch(const std::vector<PlaneTa
         if (!table.empty())
             cuda_check(cudaMemcpy(pt.table.data(), table.data(), table.size(), cudaMemcpyHostToDevice),
                        "uploading job table");
+    }
+    if (n_parts == 1) {
+        const auto &launches = b->parts[0]->compiled.launches;
+        std::size_t most[2] = {0, 0};
+        bool independent = true;
+        for (const auto &l : launches) {
+            ++most[l.pass];
+            // Refinement and its conversion follow their pass's solve.
+            independent = independent && l.kind != 7 && l.kind != 8;
+        }
+        const std::size_t n = std::max(most[0], most[1]);
+        if (independent && n >= kBranchLaunches) {
+            for (std::size_t k = 1; k < std::min(n, kMaxBranches); ++k)
+                b->branches.push_back(std::make_unique<PreparedBatch::Impl::Branch>());
+            cuda_check(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming), "creating event");
+        }
     }
     if (n_parts == 2) {
         cuda_check(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking), "creating stream");
