@@ -700,7 +700,10 @@ struct Executor::Impl {
                  const std::function<char *(std::size_t)> &scratch, std::uint32_t *status,
                  const Tuning *tuning = nullptr, int vectors_per_warp = 0);
     void launch(const Compiled &c, const char *device_table, cudaStream_t stream, std::uint32_t *status);
-    void launch(const Launch &l, const char *device_table, cudaStream_t stream, std::uint32_t *status);
+    // `follows`: the launch before this one on the stream is another of the
+    // same batch.
+    void launch(const Launch &l, const char *device_table, cudaStream_t stream, std::uint32_t *status,
+                bool follows = false);
     // `copies`: a stream holding the tasks' input copies; the job table is
     // copied behind them there and the kernels wait for both.
     void enqueue(Workspace &ws, const std::vector<PlaneTask> &tasks, char *scratch = nullptr,
@@ -1405,7 +1408,8 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
     out.tasks = tasks.size();
 }
 
-void Executor::Impl::launch(const Launch &l, const char *device_table, cudaStream_t stream, std::uint32_t *status) {
+void Executor::Impl::launch(const Launch &l, const char *device_table, cudaStream_t stream, std::uint32_t *status,
+                            bool follows) {
     Record *rec = nullptr;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(stream, &capturing);
@@ -1436,7 +1440,7 @@ void Executor::Impl::launch(const Launch &l, const char *device_table, cudaStrea
     } else if (l.kind == 5) {
         rc = l.variant & 31
             ? launch_xring(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
-                           l.variant & 31, l.per_lane, (l.variant & kTiled) != 0, l.in, l.out, stream)
+                           l.variant & 31, l.per_lane, (l.variant & kTiled) != 0, l.in, l.out, follows && !rec, stream)
             : launch_tsolve(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.threads,
                             l.hb, l.in, l.out, l.record_floats, stream);
     } else if (ring_kind(l.kind)) {
@@ -1444,7 +1448,7 @@ void Executor::Impl::launch(const Launch &l, const char *device_table, cudaStrea
                           l.variant & 31, l.per_lane,
                           l.kind == 10 ? (l.pass ? RingLayout::columns : RingLayout::rows)
                           : l.variant & kTiled ? RingLayout::tiled : RingLayout::plain,
-                          l.in, l.out, stream);
+                          l.in, l.out, follows && !rec, stream);
     } else if (l.kind == 2) {
         rc = launch_stream(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks,
                            l.hb, kStreamChunk, l.pass == 0, l.in, l.out, l.record_floats,
@@ -1462,7 +1466,7 @@ void Executor::Impl::launch(const Launch &l, const char *device_table, cudaStrea
 
 void Executor::Impl::launch(const Compiled &c, const char *device_table, cudaStream_t stream,
                             std::uint32_t *status) {
-    for (const auto &l : c.launches) launch(l, device_table, stream, status);
+    for (const auto &l : c.launches) launch(l, device_table, stream, status, &l != c.launches.data());
     std::scoped_lock lock(mutex);
     stats.launches += c.launches.size();
     stats.plane_tasks += c.tasks;

@@ -115,7 +115,8 @@ constexpr int kTRingThreads = 128;
 constexpr int kTResidentWarps = 16;    // resident warps per SM (128 registers a thread)
 constexpr int kMinSegmentChunks = 1;   // shortest segment, in chunks (StreamJob)
 int launch_tring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
-                 int per_lane, RingLayout layout, dev::Sample in, dev::Sample out, void *stream);
+                 int per_lane, RingLayout layout, dev::Sample in, dev::Sample out, bool follows,
+                 void *stream);
 
 // Columns passes with fused candidate scoring (tscore_impl.cuh): as
 // the transposing passes, for Float32 intermediates with chunk-delayed records
@@ -131,7 +132,7 @@ int launch_tscore(const dev::StreamJob *jobs, int job_count, int total_blocks, i
 // of launch_tring; launch_tsolve (tsolve_impl.cuh) serves the plans whose
 // group refill exceeds that ring.
 int launch_xring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
-                 int per_lane, bool tiled, dev::Sample in, dev::Sample out, void *stream);
+                 int per_lane, bool tiled, dev::Sample in, dev::Sample out, bool follows, void *stream);
 bool tsolve_supports(int half_bandwidth);
 int launch_tsolve(const dev::StreamJob *jobs, int job_count, int total_blocks, int threads, int half_bandwidth,
                   dev::Sample in, dev::Sample out, int record_floats, void *stream);

@@ -530,6 +530,13 @@ __device__ __forceinline__ void rstore_wait() {
     __syncwarp();
 }
 
+// Waits for the launch before this one, its results included, where this one
+// started early (StreamJob's launches, `follows`); nothing else.
+__device__ __forceinline__ void ring_launch_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+// Lets such a launch behind this one start once every CTA is past this point.
+__device__ __forceinline__ void ring_launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 template <int HB, int W, int V, RingLayout LAYOUT, class In, class Out>
 __global__ void __launch_bounds__(kRingThreads, 4 / V)
 tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
@@ -601,7 +608,9 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
               tm + (static_cast<unsigned>(warp * 32) << 16),
               static_cast<unsigned>(__cvta_generic_to_shared(ring_smem + warp * kRingBuffers * Feed::BUFFER)),
               static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][0])));
+    ring_launch_wait();
     if (!idle) feed.start(c0 > 0 ? lead.first_sample : 0);
+    ring_launch_next();
 
     Out *out[V];
 #pragma unroll
@@ -679,44 +688,61 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" :: "r"(tm), "n"(COLUMNS));
 }
 
+// A launch that may start while the stream's launch before it still runs: the
+// kernels read only their jobs and records (which that launch does not write)
+// until ring_launch_wait.
+inline cudaError_t ring_launch(void (*kernel)(const StreamJob *, int), const StreamJob *jobs, int count, int blocks,
+                               int smem, bool follows, cudaStream_t s) {
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(static_cast<unsigned>(blocks));
+    config.blockDim = dim3(kRingThreads);
+    config.dynamicSmemBytes = static_cast<std::size_t>(smem);
+    config.stream = s;
+    config.attrs = &early;
+    config.numAttrs = follows ? 1 : 0;
+    return cudaLaunchKernelEx(&config, kernel, jobs, count);
+}
+
 template <int HB, int W, int V, RingLayout LAYOUT, class In, class Out>
-int rlaunch_typed(const StreamJob *jobs, int count, int blocks, cudaStream_t s) {
+int rlaunch_typed(const StreamJob *jobs, int count, int blocks, bool follows, cudaStream_t s) {
     constexpr int smem = 1024 + 3 * RingRecord<HB, W>::CHUNK * 4
         + kRingThreads / 32 * (kRingBuffers * RingFeeder<In, V, W, LAYOUT>::BUFFER
                                + (LAYOUT == RingLayout::rows ? V * 4096 : 0));
     auto kernel = tring_kernel<HB, W, V, LAYOUT, In, Out>;
     static SmemLimit limit;
     if (const cudaError_t e = limit.ensure(kernel, smem); e != cudaSuccess) return static_cast<int>(e);
-    kernel<<<blocks, kRingThreads, smem, s>>>(jobs, count);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(ring_launch(kernel, jobs, count, blocks, smem, follows, s));
 }
 
 template <int HB, int W, int V>
 int rlaunch(const StreamJob *jobs, int count, int blocks, dev::Sample in, dev::Sample out, RingLayout layout,
-            void *stream) {
+            bool follows, void *stream) {
     using dev::Sample;
     using std::uint16_t, std::uint8_t;
     using L = RingLayout;
     const auto s = static_cast<cudaStream_t>(stream);
     if (in == Sample::f32 && out == Sample::f32) {
         switch (layout) {
-        case L::plain: return rlaunch_typed<HB, W, V, L::plain, float, float>(jobs, count, blocks, s);
-        case L::tiled: return rlaunch_typed<HB, W, V, L::tiled, float, float>(jobs, count, blocks, s);
-        case L::rows: return rlaunch_typed<HB, W, V, L::rows, float, float>(jobs, count, blocks, s);
-        case L::columns: return rlaunch_typed<HB, W, V, L::columns, float, float>(jobs, count, blocks, s);
+        case L::plain: return rlaunch_typed<HB, W, V, L::plain, float, float>(jobs, count, blocks, follows, s);
+        case L::tiled: return rlaunch_typed<HB, W, V, L::tiled, float, float>(jobs, count, blocks, follows, s);
+        case L::rows: return rlaunch_typed<HB, W, V, L::rows, float, float>(jobs, count, blocks, follows, s);
+        case L::columns: return rlaunch_typed<HB, W, V, L::columns, float, float>(jobs, count, blocks, follows, s);
         }
     }
     if (out == Sample::f32 && layout == L::tiled) {
-        if (in == Sample::u16) return rlaunch_typed<HB, W, V, L::tiled, uint16_t, float>(jobs, count, blocks, s);
-        if (in == Sample::u8) return rlaunch_typed<HB, W, V, L::tiled, uint8_t, float>(jobs, count, blocks, s);
+        if (in == Sample::u16) return rlaunch_typed<HB, W, V, L::tiled, uint16_t, float>(jobs, count, blocks, follows, s);
+        if (in == Sample::u8) return rlaunch_typed<HB, W, V, L::tiled, uint8_t, float>(jobs, count, blocks, follows, s);
     }
     if (out == Sample::f32 && layout == L::plain) {
-        if (in == Sample::u16) return rlaunch_typed<HB, W, V, L::plain, uint16_t, float>(jobs, count, blocks, s);
-        if (in == Sample::u8) return rlaunch_typed<HB, W, V, L::plain, uint8_t, float>(jobs, count, blocks, s);
+        if (in == Sample::u16) return rlaunch_typed<HB, W, V, L::plain, uint16_t, float>(jobs, count, blocks, follows, s);
+        if (in == Sample::u8) return rlaunch_typed<HB, W, V, L::plain, uint8_t, float>(jobs, count, blocks, follows, s);
     }
     if (in == Sample::f32 && layout == L::plain) {
-        if (out == Sample::u16) return rlaunch_typed<HB, W, V, L::plain, float, uint16_t>(jobs, count, blocks, s);
-        if (out == Sample::u8) return rlaunch_typed<HB, W, V, L::plain, float, uint8_t>(jobs, count, blocks, s);
+        if (out == Sample::u16) return rlaunch_typed<HB, W, V, L::plain, float, uint16_t>(jobs, count, blocks, follows, s);
+        if (out == Sample::u8) return rlaunch_typed<HB, W, V, L::plain, float, uint8_t>(jobs, count, blocks, follows, s);
     }
     return static_cast<int>(cudaErrorInvalidValue);
 }

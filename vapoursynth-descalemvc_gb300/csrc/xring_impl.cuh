@@ -97,7 +97,9 @@ xring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
               tm + (static_cast<unsigned>(warp * 32) << 16),
               static_cast<unsigned>(__cvta_generic_to_shared(ring_smem + warp * kRingBuffers * Feed::BUFFER)),
               static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][0])));
+    ring_launch_wait();
     if (!idle) feed.start(fc0 > 0 ? lead.first_sample : 0);
+    ring_launch_next();
 
     // Forward value of destination j at yp[a][j * y_elem].  Lanes past the
     // warp's last vector repeat it.  The tiled intermediate holds whole
@@ -232,37 +234,37 @@ xring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
 }
 
 template <int HB, int W, int V, bool TILED, class In, class Out>
-int xrlaunch_typed(const StreamJob *jobs, int count, int blocks, cudaStream_t s) {
+int xrlaunch_typed(const StreamJob *jobs, int count, int blocks, bool follows, cudaStream_t s) {
     using R = RingRecord<HB, W>;
     constexpr int smem = 1024 + 3 * R::GROUPS * R::GROUP * 4
         + kRingThreads / 32 * kRingBuffers * RingFeeder<In, V, W, RingLayout::plain>::BUFFER;
     auto kernel = xring_kernel<HB, W, V, TILED, In, Out>;
     static SmemLimit limit;
     if (const cudaError_t e = limit.ensure(kernel, smem); e != cudaSuccess) return static_cast<int>(e);
-    kernel<<<blocks, kRingThreads, smem, s>>>(jobs, count);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(ring_launch(kernel, jobs, count, blocks, smem, follows, s));
 }
 
 template <int HB, int W, int V>
-int xrlaunch(const StreamJob *jobs, int count, int blocks, dev::Sample in, dev::Sample out, bool tiled, void *stream) {
+int xrlaunch(const StreamJob *jobs, int count, int blocks, dev::Sample in, dev::Sample out, bool tiled,
+             bool follows, void *stream) {
     using dev::Sample;
     using std::uint16_t, std::uint8_t;
     const auto s = static_cast<cudaStream_t>(stream);
     if (out == Sample::f32) {
         if (in == Sample::f32)
-            return tiled ? xrlaunch_typed<HB, W, V, true, float, float>(jobs, count, blocks, s)
-                         : xrlaunch_typed<HB, W, V, false, float, float>(jobs, count, blocks, s);
+            return tiled ? xrlaunch_typed<HB, W, V, true, float, float>(jobs, count, blocks, follows, s)
+                         : xrlaunch_typed<HB, W, V, false, float, float>(jobs, count, blocks, follows, s);
         if (in == Sample::u16)
-            return tiled ? xrlaunch_typed<HB, W, V, true, uint16_t, float>(jobs, count, blocks, s)
-                         : xrlaunch_typed<HB, W, V, false, uint16_t, float>(jobs, count, blocks, s);
+            return tiled ? xrlaunch_typed<HB, W, V, true, uint16_t, float>(jobs, count, blocks, follows, s)
+                         : xrlaunch_typed<HB, W, V, false, uint16_t, float>(jobs, count, blocks, follows, s);
         if (in == Sample::u8)
-            return tiled ? xrlaunch_typed<HB, W, V, true, uint8_t, float>(jobs, count, blocks, s)
-                         : xrlaunch_typed<HB, W, V, false, uint8_t, float>(jobs, count, blocks, s);
+            return tiled ? xrlaunch_typed<HB, W, V, true, uint8_t, float>(jobs, count, blocks, follows, s)
+                         : xrlaunch_typed<HB, W, V, false, uint8_t, float>(jobs, count, blocks, follows, s);
     }
     if (in == Sample::f32 && out == Sample::u16)
-        return xrlaunch_typed<HB, W, V, false, float, uint16_t>(jobs, count, blocks, s);
+        return xrlaunch_typed<HB, W, V, false, float, uint16_t>(jobs, count, blocks, follows, s);
     if (in == Sample::f32 && out == Sample::u8)
-        return xrlaunch_typed<HB, W, V, false, float, uint8_t>(jobs, count, blocks, s);
+        return xrlaunch_typed<HB, W, V, false, float, uint8_t>(jobs, count, blocks, follows, s);
     return static_cast<int>(cudaErrorInvalidValue);
 }
 
