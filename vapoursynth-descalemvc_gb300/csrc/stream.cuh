@@ -104,7 +104,10 @@ constexpr int kTRingPitch = 34;
 enum class RingLayout : std::int32_t { plain, tiled, rows, columns };
 // Chunk-delayed passes, the sample ring in tensor memory (tring_impl.cuh).
 // Every job of a launch has the same window (StreamPack::ring_window) and its
-// plan view the matching records; `per_lane` vectors a lane (1 or 2), CTAs of kTRingThreads threads.
+// plan view the matching records; `per_lane` vectors a lane (1 or 2), CTAs of
+// kTRingThreads threads.  `follows`: the launch may start before the one ahead
+// of it on the stream has ended; it reads its jobs and records before it waits
+// for that one's results.
 constexpr int kTStreamThreads = 128;   // default CTA size of the two-pass kernels
 // Float64 two-pass kernels: two warps a CTA spread a launch's segments more
 // evenly over the SMs, whose FP64 units bind (4K Spline64 frames on one
@@ -115,8 +118,7 @@ constexpr int kTRingThreads = 128;
 constexpr int kTResidentWarps = 16;    // resident warps per SM (128 registers a thread)
 constexpr int kMinSegmentChunks = 1;   // shortest segment, in chunks (StreamJob)
 int launch_tring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
-                 int per_lane, RingLayout layout, dev::Sample in, dev::Sample out, bool follows,
-                 void *stream);
+                 int per_lane, RingLayout layout, dev::Sample in, dev::Sample out, bool follows, void *stream);
 
 // Columns passes with fused candidate scoring (tscore_impl.cuh): as
 // the transposing passes, for Float32 intermediates with chunk-delayed records

@@ -531,7 +531,8 @@ __device__ __forceinline__ void rstore_wait() {
 }
 
 // Waits for the launch before this one, its results included, where this one
-// started early (StreamJob's launches, `follows`); nothing else.
+// may start early (launch_tring's `follows`).  Every thread does: a launch is
+// complete only after those before it.
 __device__ __forceinline__ void ring_launch_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
 // Lets such a launch behind this one start once every CTA is past this point.
@@ -688,9 +689,10 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" :: "r"(tm), "n"(COLUMNS));
 }
 
-// A launch that may start while the stream's launch before it still runs: the
-// kernels read only their jobs and records (which that launch does not write)
-// until ring_launch_wait.
+// Launches behind the launch before it on the stream or, `follows`, while that
+// one still ends: the way to the first sample (job table, records, tensor
+// memory, barriers), up to 3 us of a pass, then runs beside it.  The kernels
+// read only what that launch does not write until ring_launch_wait.
 inline cudaError_t ring_launch(void (*kernel)(const StreamJob *, int), const StreamJob *jobs, int count, int blocks,
                                int smem, bool follows, cudaStream_t s) {
     cudaLaunchAttribute early{};
