@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 # Width, height, planes, kernel, taps, and whether both axes are descaled.
 CASES = [(48, 32, 1, "bicubic", 3, "both"), (640, 360, 3, "lanczos", 3, "both"), (700, 330, 2, "spline64", 3, "both"),
-         (1920, 1080, 6, "bilinear", 3, "both"), (640, 360, 2, "bicubic", 3, "rows"), (640, 360, 2, "lanczos", 4, "columns")]
+         (1920, 1080, 6, "bilinear", 3, "both"), (701, 333, 3, "lanczos", 3, "both"), (701, 333, 2, "bicubic", 3, "rows"),
+         (701, 333, 2, "bicubic", 3, "columns"), (640, 360, 2, "bicubic", 3, "rows"), (640, 360, 2, "lanczos", 4, "columns")]
 
 
 @pytest.mark.parametrize("w,h,planes,kernel,taps,axes", CASES)

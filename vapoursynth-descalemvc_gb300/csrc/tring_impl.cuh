@@ -242,14 +242,15 @@ struct RingFeeder {
             }
         } else {
             // Vectors that no tensor map admits (not 16-byte aligned): each
-            // lane loads its own.
+            // lane loads its own (plain loads: the launch before may still
+            // write the plane while this one starts).
 #pragma unroll
             for (int a = 0; a < V; ++a) {
                 const In *p = static_cast<const In *>(in) + (first + min(lane + 32 * a, vectors - 1)) * in_vec;
                 In vals[kRingStep];
 #pragma unroll
                 for (int i = 0; i < kRingStep; ++i)
-                    vals[i] = __ldg(p + (COLS ? min(have + i, size - 1) * in_elem : min(have + i, size - 1)));
+                    vals[i] = p[COLS ? min(have + i, size - 1) * in_elem : min(have + i, size - 1)];
 #pragma unroll
                 for (int i = 0; i < NR; ++i) {
                     unsigned w = 0;
