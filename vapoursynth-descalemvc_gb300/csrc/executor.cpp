@@ -51,6 +51,20 @@ constexpr int kSeqThreads = 128;   // threads per block of the sequential kernel
 // Prepared batches of at least this many 2D tasks (and their own scratch) run
 // as two parts on two streams.
 constexpr std::size_t kSplitBatchTasks = 8;
+// ... but not small batches of Float32 planes, which one part's segments spread
+// over the GPU: two parts each split for the whole of it, so that half the work
+// is their ranges' warm-ups.  One part where the longer pass's warps (whole
+// vectors, 32 a warp) come to at most the resident warp slots over 3 (chunk-
+// delayed kernels), over 4 (half-bandwidth 1, nearer to memory) or over 6
+// (two-pass kernels, whose margins let them split half as far).  Measured on one
+// GB300 (2432 slots), us a pass in two parts and in one, with the warps of the
+// longer pass: bicubic 24 planes of 640x360 (360) 49.7 and 31.5, 64 (960) 79.9 and
+// 54.7, 8 of 1080p (320) 80.0 and 54.4, 20 (800) 124 and 101, 24 (960) 140 and 133, 40
+// (1600) 197 and 236, 8 of 4K (640) 168 and 151, 12 (960) 229 and 245; bilinear 12 of
+// 1080p (480) 81.6 and 78.9, 16 (640) 95.2 and 99.4; Lanczos4 24 of 640x360 (360) 84.9
+// and 72.2, 8 of 1080p (320) 148 and 142, 12 (480) 180 and 213.  Integer planes keep two
+// parts: where vectors split decides their last codes.
+constexpr long kWholeSlots = 3, kWholeSlotsHb1 = 4, kWholeSlotsExact = 6;
 // Prepared batches in one part with a pass of at least this many launches
 // (plans of different kernels) run them side by side: each alone leaves most
 // SMs idle (a 1080p sweep of 189 candidates, seven launches a pass: 2418 us one
@@ -2318,6 +2332,37 @@ std::unique_ptr<PreparedBatch> Executor::prepare_batch(const std::vector<PlaneTa
         n_parts = !scratch && static_cast<std::size_t>(planes) >= kSplitBatchTasks ? 2 : 1;
     }
     if (n_parts != 1 && n_parts != 2) throw std::invalid_argument("a prepared batch has 1 or 2 parts");
+    auto add_part = [&](const std::vector<PlaneTask> &part_tasks) {
+        b->parts.push_back(std::make_unique<PreparedBatch::Impl::Part>());
+        auto &pt = *b->parts.back();
+        impl_->compile(part_tasks, pt.compiled, [&](std::size_t bytes) {
+            if (scratch) {
+                if (bytes > scratch_capacity) throw std::length_error("batch scratch exceeds the caller's buffer");
+                return static_cast<char *>(scratch);
+            }
+            pt.scratch.reserve(bytes);
+            return pt.scratch.data();
+        }, b->status, &t, vectors_per_warp);
+    };
+    if (parts == 0 && n_parts == 2 && impl_->segment_mode == 0) {
+        long warps[2] = {0, 0};
+        bool floats = true;
+        for (const auto &task : tasks) {
+            if (task.vertical) warps[0] += (task.vertical->source_size + 31) / 32;
+            if (task.horizontal) warps[1] += (task.horizontal->destination_size + 31) / 32;
+            floats = floats && task.horizontal && task.vertical && task.sample == dev::Sample::f32;
+        }
+        const long most = std::max(warps[0], warps[1]);
+        if (floats && most * kWholeSlots <= impl_->warp_slots) {
+            add_part(tasks);
+            long over = kWholeSlots;
+            for (const auto &l : b->parts[0]->compiled.launches)
+                over = std::max(over, ring_kind(l.kind) ? (l.hb == 1 ? kWholeSlotsHb1 : kWholeSlots)
+                                      : l.kind == 5 || l.kind == 6 ? kWholeSlotsExact : impl_->warp_slots + 1L);
+            if (most * over <= impl_->warp_slots) n_parts = 1;
+            else b->parts.clear();
+        }
+    }
     if (n_parts == 2 && (scratch || tasks.size() < 2))
         throw std::invalid_argument("two batch parts need two tasks and batch-owned scratch");
     std::size_t cut = tasks.size();
@@ -2336,20 +2381,15 @@ std::unique_ptr<PreparedBatch> Executor::prepare_batch(const std::vector<PlaneTa
             if (acc >= total / 2) break;
         }
     }
-    for (int k = 0; k < n_parts; ++k) {
-        b->parts.push_back(std::make_unique<PreparedBatch::Impl::Part>());
-        auto &pt = *b->parts.back();
-        const std::vector<PlaneTask> part_tasks = n_parts == 1 ? tasks
-            : k == 0 ? std::vector<PlaneTask>(tasks.begin(), tasks.begin() + static_cast<std::ptrdiff_t>(cut))
-                     : std::vector<PlaneTask>(tasks.begin() + static_cast<std::ptrdiff_t>(cut), tasks.end());
-        impl_->compile(part_tasks, pt.compiled, [&](std::size_t bytes) {
-            if (scratch) {
-                if (bytes > scratch_capacity) throw std::length_error("batch scratch exceeds the caller's buffer");
-                return static_cast<char *>(scratch);
-            }
-            pt.scratch.reserve(bytes);
-            return pt.scratch.data();
-        }, b->status, &t, vectors_per_warp);
+    if (n_parts == 2) {
+        const auto mid = tasks.begin() + static_cast<std::ptrdiff_t>(cut);
+        add_part({tasks.begin(), mid});
+        add_part({mid, tasks.end()});
+    } else if (b->parts.empty()) {
+        add_part(tasks);
+    }
+    for (const auto &part : b->parts) {
+        auto &pt = *part;
         const auto &table = pt.compiled.table;
         pt.table.reserve(std::max<std::size_t>(table.size(), 1));
         if (!table.empty())
