@@ -769,12 +769,16 @@ constexpr int kTiled = 32;
 // on the two-pass kernels with the ring in shared memory.
 int compiled_window(const DevicePlan &dp) { return dp.ring_window; }
 
-// Launches of at least this many warps an SM (at one vector a lane) run two
+// Launches of at least kPairingWarps warps an SM (at one vector a lane) run two
 // vectors a lane: a record's load then serves both, and four warps an SM stay.
-// Measured on one GB300: 64 YUV420P16 1080p frames (14 warps an SM) 546 us a
-// batch at one vector a lane, 536 at two; 32 4K Float32 frames (14) 640 and
-// 604; 24 YUV420P8 720x480 frames (4) 95.6 and 132.
-constexpr int kPairingWarps = 8;
+// In segments it takes kPairingRanges, and that the pairs' CTAs, two an SM, come to
+// no second wave.  2D passes of half-bandwidth 1, little substitution per sample,
+// run one throughout.  Measured on one GB300, us a pass at one and at two: 64
+// YUV420P16 1080p frames (14 warps an SM) 552 and 536; Float32 bicubic, 32 of 4K 561
+// and 526, eight 169 and 152, four of 1080p 40 and 35, one of 1080p (9 warps an SM in
+// ranges) 20.7 and 24.3, one of 4K (315 CTAs of pairs) 40 and 43; bilinear, one of
+// 1080p 17.3 and 18.2, twelve 61 and 79, one of 4K 32 and 40, 32 of 4K 490 and 574.
+constexpr int kPairingWarps = 8, kPairingRanges = 10;
 
 // One-axis passes in segments: two chunks of zero-history warm-up leave below
 // 2^-52 of it, so that a segment's forward values come to the whole vector's
@@ -855,15 +859,33 @@ void push_segments(std::vector<Item> &group, const Item &whole, const std::vecto
     }
 }
 
+// CTAs of four warps of `vectors` vectors that a launch of `items` takes: changes of
+// plan or chunk range round up to whole CTAs.
+template <class Item>
+long run_ctas(const std::vector<Item> &items, int vectors) {
+    long ctas = 0, warps = 0;
+    for (std::size_t i = 0; i < items.size(); ++i) {
+        const auto &j = items[i].stream;
+        if (i && (j.plan.forward != items[i - 1].stream.plan.forward || j.chunk_begin != items[i - 1].stream.chunk_begin)) {
+            ctas += (warps + 3) / 4;
+            warps = 0;
+        }
+        warps += (j.vectors + vectors - 1) / vectors;
+    }
+    return ctas + (warps + 3) / 4;
+}
+
 // Jobs of a chunk-delayed transposing launch group (sorted by plan), split
 // into segments of whole chunks.  Automatic mode: when the group's warps fill
 // fewer than `slots` resident warp slots, up to slots / warps segments per
 // job; each segment spans at least kMinSegmentChunks chunks, and only plans
 // whose forward warm-up is admitted split.  Per plan, the jobs come segment
 // by segment, so that only plan and segment changes round up to whole CTAs.
+// `pairs`: no more segments than leave the launch in one wave at two vectors a
+// lane (a lone 4K bicubic plane: 35 segments 43 us, 30 36).
 template <class Item>
 std::vector<Item> segment_items(const std::vector<Item> &items, int vectors_per_warp, int mode, int slots, int margin = 1,
-                                int shortest = kMinSegmentChunks) {
+                                int shortest = kMinSegmentChunks, bool pairs = false) {
     if (mode == 1) return items;
     int segments = mode;
     if (mode == 0) {
@@ -871,6 +893,8 @@ std::vector<Item> segment_items(const std::vector<Item> &items, int vectors_per_
         for (const auto &it : items) warps += (it.stream.vectors + vectors_per_warp - 1) / vectors_per_warp;
         if (warps <= 0 || slots <= 0) return items;
         segments = static_cast<int>(std::min<long>(slots / warps, 64));
+        if (const long fit = slots / 8 / run_ctas(items, 64); pairs && fit >= 2 && fit < segments)
+            segments = static_cast<int>(fit);
         if (segments < 2) return items;
     }
     std::vector<Item> out;
@@ -1368,13 +1392,23 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
         } else if (ring) {
             // The split does not depend on the vectors a lane: neither do the
             // results.
-            if (key.kind == 3) items = segment_items(items, 32, segment_mode, warp_slots);
+            const std::size_t whole = items.size();
+            const bool floats = key.in == dev::Sample::f32 && key.out == dev::Sample::f32;
+            if (key.kind == 3)
+                items = segment_items(items, 32, segment_mode, warp_slots, 1, kMinSegmentChunks, floats && key.hb > 1);
             if (key.kind == 10)
                 items = segment_items(items, 32, segment_mode, warp_slots, kAxisMargin, kAxisMinChunks);
             long warps = 0;
             for (const auto &it : items) warps += (it.stream.vectors + 31) / 32;
-            if (!vectors_per_warp && warps >= kPairingWarps * static_cast<long>(warp_slots / kTResidentWarps))
-                per_lane = 2;
+            const long sms = warp_slots / kTResidentWarps;
+            bool pair = warps >= kPairingWarps * sms;
+            if (key.kind == 3) {
+                const bool ranges = items.size() > whole;
+                pair = pair && key.hb > 1
+                    && !(ranges && (warps < kPairingRanges * sms
+                                    || (warp_slots / 8 < run_ctas(items, 64) && run_ctas(items, 32) <= warp_slots / 4)));
+            }
+            if (!vectors_per_warp && pair) per_lane = 2;
         }
         if (ring)
             for (auto &it : items) {
