@@ -10,7 +10,8 @@
 //    tensor map per plane, 128-byte swizzle) into one of the warp's two
 //    staging buffers, completed on that buffer's mbarrier; the next block is
 //    in flight while the current one is consumed.  The swizzle lets a lane
-//    read its own vectors without bank conflicts.  Every wait is bounded.
+//    read its own vectors without bank conflicts.  Every wait is bounded.  Rows
+//    that no tensor map admits come word by word (copy_words).
 //  * Ring: a lane converts 16 samples of its vectors at a time to float and
 //    stores them to tensor memory (lane = vector, column = sample mod 48, the
 //    first 16 columns again after the ring so that every window of up to 16
@@ -102,6 +103,12 @@ template <class T> __device__ __forceinline__ T rout(float v, const Conversion &
 
 // ---- ring feeder ---------------------------------------------------------------
 
+// Arrivals that complete a block: of vectors that no tensor map admits (not 16-byte
+// aligned) every lane copies its words.  A stall test expects one that nothing makes.
+template <RingLayout LAYOUT> __device__ __forceinline__ unsigned ring_arrivals(const StreamJob &j, const StreamJob &lead) {
+    return (LAYOUT == RingLayout::columns || j.mapped ? 1 : 32) + (lead.feed_stall_test ? 1 : 0);
+}
+
 // LAYOUT columns: a vector's samples are a plane's column.
 template <class In, int V, int W, RingLayout LAYOUT>
 struct RingFeeder {
@@ -113,9 +120,8 @@ struct RingFeeder {
     static constexpr int BUFFER = 32 * V * 128;                     // bytes per staging buffer
     static constexpr int NR = kRingStep * static_cast<int>(sizeof(In)) / 4;   // words of a step's samples
 
-    const void *in;          // the plane
-    std::int64_t in_vec, in_elem;
-    std::uint64_t map;       // its tensor map, 0: vectors not 16-byte aligned
+    const StreamJob *job;
+    std::uint64_t map;       // the plane's tensor map, 0: vectors not 16-byte aligned
     int first;               // the warp's first vector
     int vectors;             // its valid vectors (>= 1)
     int size;                // samples per vector
@@ -137,9 +143,7 @@ struct RingFeeder {
     // `stage_at`, `mbar_at`: the warp's staging buffers and their barriers.
     __device__ __forceinline__ void init(const StreamJob &j, int samples, int first_vector, int count_vectors, int l,
                                          unsigned ring_at, unsigned stage_at, unsigned mbar_at) {
-        in = j.in;
-        in_vec = j.in_vec;
-        in_elem = j.in_elem;
+        job = &j;
         map = j.mapped ? reinterpret_cast<std::uint64_t>(j.map) : 0;
         first = first_vector;
         vectors = count_vectors;
@@ -164,8 +168,75 @@ struct RingFeeder {
         __syncwarp();
     }
 
+    // The block at `next` of `count` vectors from `first` on without a tensor map: a
+    // word a lane, 128 contiguous bytes a warp-wide copy, where TMA would put it, zeros
+    // past the vectors' end.  By cp.async where the vectors begin at a word.  A lane
+    // loading its own vector's next 16 samples, unstaged, waited on memory at each
+    // step: one GB300, eight 1919x1079 Float32 planes' rows 219 -> 80 us, sixteen 1079x607
+    // planes 67 -> 53, 24 YUV420P8 frames of 720x480 with tight rows 90 -> 80 (a lone frame
+    // of 8-bit rows that begin inside a word 23 -> 26: its copies wait), and without
+    // those loads in every refill 64 aligned YUV420P16 1080p frames 536 -> 526.
+    static __device__ __noinline__ void copy_words(const StreamJob *job, int first, int next, int size, int count,
+                                                   unsigned to, unsigned mb) {
+        constexpr int PER = 4 / static_cast<int>(sizeof(In));      // samples a word
+        const int lane = threadIdx.x & 31, at = next + lane * PER;
+        const int samples = max(min(PER, size - at), 0);
+        const std::int64_t vec = job->in_vec;
+        const In *plane = static_cast<const In *>(job->in);
+        const In *p = plane + first * vec + (samples ? at : next);
+        auto put = [&](int v) { return to + v * 128 + (((lane >> 2) ^ (v & 7)) * 16) + (lane & 3) * 4; };
+        if (PER == 1 || ((reinterpret_cast<std::uint64_t>(plane) | static_cast<std::uint64_t>(vec) * sizeof(In)) & 3) == 0) {
+#pragma unroll 8
+            for (int v = 0; v < count; ++v, p += vec)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n"
+                             :: "r"(put(v)), "l"(p), "r"(samples * static_cast<int>(sizeof(In))) : "memory");
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" :: "r"(mb) : "memory");
+        } else {
+            // Vectors that begin inside a word: the samples of BATCH in flight
+            // at a time, loaded without a branch (repeats past the ends).  Plain
+            // loads: the launch before may still write the plane while this
+            // one starts.
+            constexpr int BATCH = 32 / PER;
+            const In *row0 = plane + first * vec;
+            int column[PER];
+            unsigned mask = 0;
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                column[k] = min(at + k, size - 1);
+                if (k < samples) mask |= (0xffffffffu >> (32 - 32 / PER)) << (k * 32 / PER);
+            }
+#pragma unroll 1
+            for (int v = 0; v < count; v += BATCH) {
+                In x[BATCH][PER];
+#pragma unroll
+                for (int i = 0; i < BATCH; ++i) {
+                    const In *r = row0 + min(v + i, count - 1) * vec;
+#pragma unroll
+                    for (int k = 0; k < PER; ++k) x[i][k] = r[column[k]];
+                }
+#pragma unroll
+                for (int i = 0; i < BATCH; ++i) {
+                    unsigned w = 0;
+#pragma unroll
+                    for (int k = 0; k < PER; ++k) w |= static_cast<unsigned>(x[i][k]) << (k * 32 / PER);
+                    if (v + i < count) asm volatile("st.shared.u32 [%0], %1;\n" :: "r"(put(v + i)), "r"(w & mask) : "memory");
+                }
+            }
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" :: "r"(mb) : "memory");
+        }
+    }
+
     // Fetches the block at `next` into buffer `slot`.
     __device__ __forceinline__ void issue(unsigned slot) {
+        if constexpr (!COLS) {
+            if (!map) {
+                if (next < limit)
+                    copy_words(job, first, next, size, vectors, stage + slot * BUFFER, mbar + slot * 8);
+                __syncwarp();
+                next += SB;
+                return;
+            }
+        }
         unsigned elected;
         asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(elected));
         if (elected && next < limit) {
@@ -210,60 +281,47 @@ struct RingFeeder {
     // Waits for the copies still in flight (the block being consumed and the
     // next): none writes to shared memory after the CTA has ended.
     __device__ __forceinline__ void drain() const {
-        if (map)
+        if (!COLS || map)
             for (int k = max(count - 1, 0), from = next - (count - k + 1) * SB; k <= count; ++k, from += SB)
                 if (from < size) wait(k);
     }
 
     // Loads the next step's samples of every vector.
     __device__ __forceinline__ void fetch(unsigned (&raw)[V][NR]) {
-        if (map) {
-            if (have % SB == 0) enter();
-            if constexpr (COLS) {
-                // [sample][column]: one load a sample.
-#pragma unroll
-                for (int a = 0; a < V; ++a)
-#pragma unroll
-                    for (int i = 0; i < NR; ++i)
-                        asm volatile("ld.shared.u32 %0, [%1];"
-                                     : "=r"(raw[a][i]) : "r"(at + row[a] + (have % SB + i) * (128 * V)));
-                return;
-            }
-            // 16-byte pieces lie in the tensor map's 128-byte swizzle.
-            const unsigned piece = (have % SB) / SPL;
+        if (COLS && !map) {
+            // Columns that no tensor map admits: each lane loads its own (plain
+            // loads: the launch before may still write the plane while this one
+            // starts).
 #pragma unroll
             for (int a = 0; a < V; ++a) {
+                const float *p = static_cast<const float *>(job->in) + first + min(lane + 32 * a, vectors - 1);
+                const std::int64_t elem = job->in_elem;
 #pragma unroll
-                for (int i = 0; i < NR / 4; ++i)
-                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                                 : "=r"(raw[a][4 * i]), "=r"(raw[a][4 * i + 1]), "=r"(raw[a][4 * i + 2]),
-                                   "=r"(raw[a][4 * i + 3])
-                                 : "r"(at + (row[a] ^ ((piece + i) * 16))));
+                for (int i = 0; i < NR; ++i) raw[a][i] = __float_as_uint(p[min(have + i, size - 1) * elem]);
             }
-        } else {
-            // Vectors that no tensor map admits (not 16-byte aligned): each
-            // lane loads its own (plain loads: the launch before may still
-            // write the plane while this one starts).
+            return;
+        }
+        if (have % SB == 0) enter();
+        if constexpr (COLS) {
+            // [sample][column]: one load a sample.
 #pragma unroll
-            for (int a = 0; a < V; ++a) {
-                const In *p = static_cast<const In *>(in) + (first + min(lane + 32 * a, vectors - 1)) * in_vec;
-                In vals[kRingStep];
+            for (int a = 0; a < V; ++a)
 #pragma unroll
-                for (int i = 0; i < kRingStep; ++i)
-                    vals[i] = p[COLS ? min(have + i, size - 1) * in_elem : min(have + i, size - 1)];
+                for (int i = 0; i < NR; ++i)
+                    asm volatile("ld.shared.u32 %0, [%1];"
+                                 : "=r"(raw[a][i]) : "r"(at + row[a] + (have % SB + i) * (128 * V)));
+            return;
+        }
+        // 16-byte pieces lie in the tensor map's 128-byte swizzle.
+        const unsigned piece = (have % SB) / SPL;
 #pragma unroll
-                for (int i = 0; i < NR; ++i) {
-                    unsigned w = 0;
-                    if constexpr (sizeof(In) == 4) {
-                        w = __float_as_uint(vals[i]);
-                    } else {
-                        constexpr int N = 4 / static_cast<int>(sizeof(In));
+        for (int a = 0; a < V; ++a) {
 #pragma unroll
-                        for (int k = 0; k < N; ++k) w |= static_cast<unsigned>(vals[i * N + k]) << (k * 32 / N);
-                    }
-                    raw[a][i] = w;
-                }
-            }
+            for (int i = 0; i < NR / 4; ++i)
+                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(raw[a][4 * i]), "=r"(raw[a][4 * i + 1]), "=r"(raw[a][4 * i + 2]),
+                               "=r"(raw[a][4 * i + 3])
+                             : "r"(at + (row[a] ^ ((piece + i) * 16))));
         }
     }
 
@@ -276,7 +334,7 @@ struct RingFeeder {
         column = from % kRingColumns;
         count = 0;
         next = from / SB * SB;
-        if (map) {
+        if (!COLS || map) {
             issue(0);
             if (from % SB) enter();
         }
@@ -591,8 +649,7 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
     }
     if (lane < kRingBuffers) {
         const unsigned mb = static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][lane]));
-        // A stall test expects an arrival that nothing makes.
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" :: "r"(mb), "r"(lead.feed_stall_test ? 2 : 1) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" :: "r"(mb), "r"(ring_arrivals<LAYOUT>(job, lead)) : "memory");
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n");

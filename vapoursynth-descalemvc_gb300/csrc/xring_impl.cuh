@@ -80,8 +80,7 @@ xring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
     }
     if (lane < kRingBuffers) {
         const unsigned mb = static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][lane]));
-        // A stall test expects an arrival that nothing makes.
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" :: "r"(mb), "r"(lead.feed_stall_test ? 2 : 1) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" :: "r"(mb), "r"(ring_arrivals<RingLayout::plain>(job, lead)) : "memory");
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n");
