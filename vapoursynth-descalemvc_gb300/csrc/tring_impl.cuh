@@ -39,11 +39,11 @@
 //    in two sums), chunk-delayed backward substitution with a zero-carry
 //    warm-up over the following chunk.  Every rounding is the same for any V.
 //
-// What bounds them: instruction issue (53 instructions per 32 results at one
-// vector a lane, 0.62 of the issue slots busy) beside the shared-memory pipe
-// (14.5 cycles per 32 results, 61 % busy).  Measured on one GB300 against the
+// What bounds them: instruction issue and dependent FMA chains (43-50 % of the
+// slots busy at two vectors a lane, 56-64 % on the busiest SM), the shared-memory
+// pipe no longer (25-33 %, 70-76 % before).  Measured on one GB300 against the
 // kernels with both in registers and shared memory: 64 YUV420P16 1080p frames
-// to 810p 769 -> 536 us, 32 4K Float32 frames to 1440p 1017 -> 604 us.
+// to 810p 769 -> 526 us, 32 4K Float32 frames to 1440p 1017 -> 580 us.
 #pragma once
 
 #include "tstream_impl.cuh"
