@@ -2312,7 +2312,10 @@ std::size_t Executor::batch_scratch_bound(const std::vector<PlaneTask> &tasks) {
         const bool f64 = (h && h->requires_float64()) || (v && v->requires_float64());
         const std::size_t es = f64 ? 8 : 4;
         const std::size_t hd = h ? static_cast<std::size_t>(h->destination_size) : static_cast<std::size_t>(t.vectors);
-        const std::size_t vs = v ? (static_cast<std::size_t>(v->source_size) + 3) / 4 * 4 : static_cast<std::size_t>(t.vectors);
+        // Tiled intermediates hold whole tiles of 32 rows; the bound on the forward values
+        // below covers what that adds, but for outputs of a single chunk of rows.
+        const std::size_t whole = v && h && v->destination_size <= kStreamChunk ? 32 : 4;
+        const std::size_t vs = v ? (static_cast<std::size_t>(v->source_size) + whole - 1) / whole * whole : static_cast<std::size_t>(t.vectors);
         const std::size_t vd = v ? static_cast<std::size_t>(v->destination_size) : static_cast<std::size_t>(t.vectors);
         bytes += align_up(hd * vs * es) + (t.score ? 0 : align_up(hd * vd * es));
         if (h && v) {
