@@ -255,6 +255,25 @@ int dsmvc_gb_plan_stream_info(const dsmvc_gb_plan *plan,
  * per four destinations, group_stride floats each, whole chunks); `count`
  * receives the floats needed, `out` may be NULL to query it. */
 int dsmvc_gb_plan_stream_groups(const dsmvc_gb_plan *plan, float *out, uint64_t capacity, uint64_t *count);
+/* The records of the kernels with the sample ring in tensor memory (window 0
+ * and no records where they do not admit the plan), one group per four
+ * destinations, whole chunks.  Forward: the four windows' ring columns (int32
+ * bits; the first word also holds, above bit 8, the end of the group's last
+ * window in blocks of 16 samples, rounded up), four inverse diagonals, the four
+ * windows' weights, the four destinations' lower factors; backward: their
+ * backward factors (both padded to 4).  `first_blocks`: per chunk of
+ * destinations, the sample at which a range starting there begins its ring.
+ * The buffers may be NULL to query the counts. */
+typedef struct dsmvc_gb_stream_ring {
+    int32_t window;              /* compiled gather window */
+    int32_t columns;             /* samples the ring holds */
+    uint64_t forward_count, backward_count, first_blocks_count;
+} dsmvc_gb_stream_ring;
+int dsmvc_gb_plan_stream_ring(const dsmvc_gb_plan *plan,
+                              dsmvc_gb_stream_ring *info, float *forward,
+                              uint64_t forward_capacity, float *backward,
+                              uint64_t backward_capacity, int32_t *first_blocks,
+                              uint64_t first_blocks_capacity);
 /* planner_cache_stats / clear_planner_caches (engine.hpp:179-180). */
 int dsmvc_gb_planner_cache_stats(dsmvc_gb_planner_stats *out);
 void dsmvc_gb_clear_planner_caches(void);

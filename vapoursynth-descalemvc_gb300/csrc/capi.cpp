@@ -361,6 +361,31 @@ int dsmvc_gb_plan_stream_groups(const dsmvc_gb_plan *plan, float *out, uint64_t 
     });
 }
 
+int dsmvc_gb_plan_stream_ring(const dsmvc_gb_plan *plan, dsmvc_gb_stream_ring *info, float *forward,
+                              uint64_t forward_capacity, float *backward, uint64_t backward_capacity,
+                              int32_t *first_blocks, uint64_t first_blocks_capacity) {
+    return guarded([&] {
+        const auto &p = plan_of(plan);
+        if (!info) throw std::invalid_argument("output is null");
+        const auto pack = dsmvc_gb::pack_stream_plan(p, dsmvc_gb::kStreamChunk, dsmvc_gb::kStreamRing,
+                                                     dsmvc_gb::stream_supports(p.half_bandwidth),
+                                                     dsmvc_gb::tsolve_supports(p.half_bandwidth));
+        *info = {};
+        info->window = pack.ring_window;
+        info->columns = dsmvc_gb::kRingColumns;
+        info->forward_count = pack.ring_forward.size();
+        info->backward_count = pack.ring_backward.size();
+        info->first_blocks_count = pack.ring_first_block.size();
+        if ((forward && forward_capacity < pack.ring_forward.size())
+            || (backward && backward_capacity < pack.ring_backward.size())
+            || (first_blocks && first_blocks_capacity < pack.ring_first_block.size()))
+            throw std::length_error("ring record buffer too small");
+        if (forward) std::copy(pack.ring_forward.begin(), pack.ring_forward.end(), forward);
+        if (backward) std::copy(pack.ring_backward.begin(), pack.ring_backward.end(), backward);
+        if (first_blocks) std::copy(pack.ring_first_block.begin(), pack.ring_first_block.end(), first_blocks);
+    });
+}
+
 int dsmvc_gb_planner_cache_stats(dsmvc_gb_planner_stats *out) {
     return guarded([&] {
         if (!out) throw std::invalid_argument("output is null");

@@ -45,7 +45,8 @@ bool ring_fits_grouped(const std::vector<int> &s0, int window, int size, int rin
 
 } // namespace
 
-int ring_window(int half_bandwidth, int window) {
+int ring_window(int half_bandwidth, int window, int source_size) {
+    if (source_size > kRingMaxSource) return 0;
     // Half-bandwidth 1 windows are 4 samples below a ratio of 1.5; wider
     // kernels' never are.
     if (half_bandwidth > 7) return window <= 16 ? 16 : 0;
@@ -285,7 +286,7 @@ StreamPack pack_stream_plan(const AxisPlan &p, int chunk, int ring, bool hb_supp
     out.chunk_first_block.resize(static_cast<std::size_t>(chunks));
     for (int k = 0; k < chunks; ++k) out.chunk_first_block[static_cast<std::size_t>(k)] = s0[static_cast<std::size_t>(k) * chunk] / 16 * 16;
 
-    const int rw = (delayed && out.ring_ok_transposed) || out.exact ? ring_window(hb, window) : 0;
+    const int rw = (delayed && out.ring_ok_transposed) || out.exact ? ring_window(hb, window, m) : 0;
     if (rw) {
         // Replay of the refills: sixteen samples at a time, up to the end of
         // the group's last window.  (A source shorter than the compiled
@@ -309,7 +310,7 @@ StreamPack pack_stream_plan(const AxisPlan &p, int chunk, int ring, bool hb_supp
                 float *b = out.ring_backward.data() + j / 4 * low_floats;
                 const std::size_t q = j % 4, h = static_cast<std::size_t>(hb);
                 int head = start_of(j) % kRingColumns;
-                if (q == 0) head |= end_of(j + 3) << 8;
+                if (q == 0) head |= static_cast<int>(static_cast<unsigned>((end_of(j + 3) + 15) / 16) << 8);
                 std::memcpy(&f[q], &head, sizeof(int));
                 const float *r = out.forward.data() + j * static_cast<std::size_t>(out.forward_stride);
                 f[4 + q] = r[1];

@@ -67,9 +67,10 @@ struct StreamPack {
     // window is ring_window(hb, window) samples, starting at most at
     // source_size - ring_window.  Per group of four destinations: their four
     // ring columns (start mod kRingColumns), the first word also holding the refill
-    // target (the group's last window's end) above bit 8; the four inverse
-    // diagonals; the four windows' weights; the four destinations' lower
-    // factors back to back (use order d = hb..1), padded to 4.  Backward:
+    // target (the group's last window's end, in blocks of 16 samples, rounded
+    // up: the ring is refilled a block at a time) in the 24 bits above bit 8; the
+    // four inverse diagonals; the four windows' weights; the four destinations'
+    // lower factors back to back (use order d = hb..1), padded to 4.  Backward:
     // the four destinations' hb factors back to back, padded to 4.
     int ring_window = 0;            // 0 when not admitted
     std::vector<float> ring_forward;
@@ -77,9 +78,12 @@ struct StreamPack {
     std::vector<int> ring_first_block;   // as chunk_first_block, for these windows
 };
 
+// Longest source that the refill target's field can count.
+constexpr int kRingMaxSource = 1 << 28;
+
 // The compiled window that serves a plan's window in the kernels with the
 // ring in tensor memory; 0 when none does.
-int ring_window(int half_bandwidth, int window);
+int ring_window(int half_bandwidth, int window, int source_size);
 
 // `chunk` destinations per register chunk, `ring` source samples held per
 // thread.  A plan is eligible when its half-bandwidth has a kernel, its

@@ -375,7 +375,8 @@ struct RingFeeder {
         column = column + kRingStep == kRingColumns ? 0 : column + kRingStep;
     }
 
-    // Makes samples [0, need) resident (need <= size).
+    // Makes samples [0, need) resident (`need`: a multiple of 16, less than 16
+    // past the size).
     __device__ __forceinline__ void ensure(int need) {
         if (have >= need) return;
         do step(); while (have < need);
@@ -387,7 +388,7 @@ struct RingFeeder {
 
 // Records (StreamPack::ring_forward, ring_backward): per group of four
 // destinations, four ring columns (the first word also holds the refill
-// target above bit 8), the four inverse diagonals, the four windows' weights,
+// target, in blocks of 16 samples, above bit 8), the four inverse diagonals, the four windows' weights,
 // and the four destinations' lower factors back to back; the four
 // destinations' backward factors back to back.
 template <int HB, int W> struct RingRecord {
@@ -435,7 +436,7 @@ __device__ __forceinline__ void rforward(float (&hist)[V][HB], const float *fwd,
         for (int t = 0; t < G; t += 4) {
             const float *gr = fwd + ((tg + t) / 4) * R::GROUP;
             const int4 h = *reinterpret_cast<const int4 *>(gr);
-            feed.ensure(h.x >> 8);
+            feed.ensure(static_cast<int>(static_cast<unsigned>(h.x) >> 8) * kRingStep);
             const unsigned at[4] = {feed.ring + (h.x & 255), feed.ring + h.y, feed.ring + h.z, feed.ring + h.w};
             float x[2][V][W];
 #pragma unroll

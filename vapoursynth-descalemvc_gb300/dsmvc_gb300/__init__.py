@@ -108,6 +108,11 @@ class StreamInfoC(C.Structure):
                 ("exact_margin", C.c_int32), ("exact_margin_transfer", C.c_double)]
 
 
+class StreamRingC(C.Structure):
+    _fields_ = [("window", C.c_int32), ("columns", C.c_int32), ("forward_count", C.c_uint64),
+                ("backward_count", C.c_uint64), ("first_blocks_count", C.c_uint64)]
+
+
 class SweepOptionsC(C.Structure):
     _fields_ = [("memory_budget", C.c_int64), ("autotune", C.c_int32), ("graph", C.c_int32),
                 ("fused_scoring", C.c_int32), ("reserved", C.c_int32)]
@@ -164,6 +169,8 @@ SIGNATURES = {
     "dsmvc_gb_plan_stream_info": ([C.c_void_p, C.POINTER(StreamInfoC), C.c_void_p, C.c_uint64,
                                    C.c_void_p, C.c_uint64], C.c_int),
     "dsmvc_gb_plan_stream_groups": ([C.c_void_p, C.c_void_p, C.c_uint64, C.POINTER(C.c_uint64)], C.c_int),
+    "dsmvc_gb_plan_stream_ring": ([C.c_void_p, C.POINTER(StreamRingC), C.c_void_p, C.c_uint64, C.c_void_p,
+                                   C.c_uint64, C.c_void_p, C.c_uint64], C.c_int),
     "dsmvc_gb_planner_cache_stats": ([C.POINTER(PlannerStatsC)], C.c_int),
     "dsmvc_gb_clear_planner_caches": ([], None),
     "dsmvc_gb_executor_create": ([C.c_int32, C.POINTER(C.c_void_p)], C.c_int),
@@ -367,6 +374,21 @@ class AxisPlan:
                 _check(lib().dsmvc_gb_plan_stream_groups(self._h, groups.ctypes.data, groups.size, C.byref(count)))
                 out["groups"] = groups.reshape(-1, info.group_stride)
         return out
+
+    def stream_ring(self) -> dict:
+        """Packed records of the kernels with the ring in tensor memory
+        (dsmvc_gb_plan_stream_ring); `window` 0 where they do not admit the plan."""
+        info = StreamRingC()
+        _check(lib().dsmvc_gb_plan_stream_ring(self._h, C.byref(info), None, 0, None, 0, None, 0))
+        fwd = np.zeros(info.forward_count, np.float32)
+        bwd = np.zeros(info.backward_count, np.float32)
+        first = np.zeros(info.first_blocks_count, np.int32)
+        if info.window:
+            _check(lib().dsmvc_gb_plan_stream_ring(self._h, C.byref(info), fwd.ctypes.data, fwd.size,
+                                                   bwd.ctypes.data, bwd.size, first.ctypes.data, first.size))
+        groups = info.first_blocks_count * 8 or 1          # four destinations each, chunks of 32
+        return {"window": info.window, "columns": info.columns, "forward": fwd.reshape(groups, -1),
+                "backward": bwd.reshape(groups, -1), "first_blocks": first}
 
     def hashes(self):
         f, c = C.c_uint64(), C.c_uint64()
