@@ -717,14 +717,11 @@ struct Executor::Impl {
     // may start while what is ahead of it on the stream ends.
     void launch(const Compiled &c, const char *device_table, cudaStream_t stream, std::uint32_t *status,
                 bool resident = false);
-    // `follows`: nothing ahead of this launch on the stream writes its jobs or
-    // records, so that the ring kernels may start while it ends.  One Float32
-    // frame of 48x32, 640x360, 1920x1080 and 3840x2160 on one GB300, frames
-    // behind one another: 12.3, 24.6, 30.8 and 53.2 us with every launch
-    // behind the end of the one before, 10.3, 20.5, 26.7 and 47.3 us with
-    // only the first, 7.9, 16.2, 24.2 and 43.0 us with none.
+    // `ahead`: what is ahead of this launch on the stream; unless it has ended, it
+    // does not write this one's jobs or records, and the ring kernels may start
+    // while it ends (figures at ring_launch).
     void launch(const Launch &l, const char *device_table, cudaStream_t stream, std::uint32_t *status,
-                bool follows = false);
+                RingAhead ahead = RingAhead::ended);
     // `copies`: a stream holding the tasks' input copies; the job table is
     // copied behind them there and the kernels wait for both.
     void enqueue(Workspace &ws, const std::vector<PlaneTask> &tasks, char *scratch = nullptr,
@@ -1464,7 +1461,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
 }
 
 void Executor::Impl::launch(const Launch &l, const char *device_table, cudaStream_t stream, std::uint32_t *status,
-                            bool follows) {
+                            RingAhead ahead) {
     Record *rec = nullptr;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(stream, &capturing);
@@ -1479,6 +1476,7 @@ void Executor::Impl::launch(const Launch &l, const char *device_table, cudaStrea
         cuda_check(cudaEventRecord(rec->start, stream), "recording event");
     }
     const char *dev_table = device_table + l.offset;
+    if (rec) ahead = RingAhead::ended;
     int rc = 0;
     if (l.kind == 9) {
         rc = launch_tscore(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
@@ -1495,7 +1493,7 @@ void Executor::Impl::launch(const Launch &l, const char *device_table, cudaStrea
     } else if (l.kind == 5) {
         rc = l.variant & 31
             ? launch_xring(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.hb,
-                           l.variant & 31, l.per_lane, (l.variant & kTiled) != 0, l.in, l.out, follows && !rec, stream)
+                           l.variant & 31, l.per_lane, (l.variant & kTiled) != 0, l.in, l.out, ahead, stream)
             : launch_tsolve(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks, l.threads,
                             l.hb, l.in, l.out, l.record_floats, stream);
     } else if (ring_kind(l.kind)) {
@@ -1503,7 +1501,7 @@ void Executor::Impl::launch(const Launch &l, const char *device_table, cudaStrea
                           l.variant & 31, l.per_lane,
                           l.kind == 10 ? (l.pass ? RingLayout::columns : RingLayout::rows)
                           : l.variant & kTiled ? RingLayout::tiled : RingLayout::plain,
-                          l.in, l.out, follows && !rec, stream);
+                          l.in, l.out, ahead, stream);
     } else if (l.kind == 2) {
         rc = launch_stream(reinterpret_cast<const dev::StreamJob *>(dev_table), l.count, l.blocks,
                            l.hb, kStreamChunk, l.pass == 0, l.in, l.out, l.record_floats,
@@ -1521,7 +1519,11 @@ void Executor::Impl::launch(const Launch &l, const char *device_table, cudaStrea
 
 void Executor::Impl::launch(const Compiled &c, const char *device_table, cudaStream_t stream,
                             std::uint32_t *status, bool resident) {
-    for (const auto &l : c.launches) launch(l, device_table, stream, status, resident || &l != c.launches.data());
+    RingAhead ahead = resident ? RingAhead::any : RingAhead::ended;
+    for (const auto &l : c.launches) {
+        launch(l, device_table, stream, status, ahead);
+        ahead = RingAhead::own;
+    }
     std::scoped_lock lock(mutex);
     stats.launches += c.launches.size();
     stats.plane_tasks += c.tasks;

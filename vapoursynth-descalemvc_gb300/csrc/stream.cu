@@ -78,88 +78,88 @@ int launch_tsolve(const dev::StreamJob *jobs, int job_count, int total_blocks, i
     }
 }
 
-int launch_tring_hb1_w4(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, bool, void *);
-int launch_tring_hb1_w8(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, bool, void *);
-int launch_tring_hb1_w16(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, bool, void *);
-int launch_tring_hb3_w8(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, bool, void *);
-int launch_tring_hb3_w12(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, bool, void *);
-int launch_tring_hb3_w16(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, bool, void *);
-int launch_tring_hb5_w8(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, bool, void *);
-int launch_tring_hb5_w12(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, bool, void *);
-int launch_tring_hb5_w16(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, bool, void *);
-int launch_tring_hb7_w12(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, bool, void *);
-int launch_tring_hb7_w16(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, bool, void *);
+int launch_tring_hb1_w4(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_tring_hb1_w8(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_tring_hb1_w16(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_tring_hb3_w8(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_tring_hb3_w12(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_tring_hb3_w16(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_tring_hb5_w8(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_tring_hb5_w12(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_tring_hb5_w16(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_tring_hb7_w12(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_tring_hb7_w16(const dev::StreamJob *, int, int, int, RingLayout, dev::Sample, dev::Sample, RingAhead, void *);
 
 int launch_tring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
-                 int per_lane, RingLayout layout, dev::Sample in, dev::Sample out, bool follows,
+                 int per_lane, RingLayout layout, dev::Sample in, dev::Sample out, RingAhead ahead,
                  void *stream) {
     if (half_bandwidth == 1 && window == 4)
-        return launch_tring_hb1_w4(jobs, job_count, total_blocks, per_lane, layout, in, out, follows, stream);
+        return launch_tring_hb1_w4(jobs, job_count, total_blocks, per_lane, layout, in, out, ahead, stream);
     if (half_bandwidth == 1 && window == 8)
-        return launch_tring_hb1_w8(jobs, job_count, total_blocks, per_lane, layout, in, out, follows, stream);
+        return launch_tring_hb1_w8(jobs, job_count, total_blocks, per_lane, layout, in, out, ahead, stream);
     if (half_bandwidth == 1 && window == 16)
-        return launch_tring_hb1_w16(jobs, job_count, total_blocks, per_lane, layout, in, out, follows, stream);
+        return launch_tring_hb1_w16(jobs, job_count, total_blocks, per_lane, layout, in, out, ahead, stream);
     if (half_bandwidth == 3 && window == 8)
-        return launch_tring_hb3_w8(jobs, job_count, total_blocks, per_lane, layout, in, out, follows, stream);
+        return launch_tring_hb3_w8(jobs, job_count, total_blocks, per_lane, layout, in, out, ahead, stream);
     if (half_bandwidth == 3 && window == 12)
-        return launch_tring_hb3_w12(jobs, job_count, total_blocks, per_lane, layout, in, out, follows, stream);
+        return launch_tring_hb3_w12(jobs, job_count, total_blocks, per_lane, layout, in, out, ahead, stream);
     if (half_bandwidth == 3 && window == 16)
-        return launch_tring_hb3_w16(jobs, job_count, total_blocks, per_lane, layout, in, out, follows, stream);
+        return launch_tring_hb3_w16(jobs, job_count, total_blocks, per_lane, layout, in, out, ahead, stream);
     if (half_bandwidth == 5 && window == 8)
-        return launch_tring_hb5_w8(jobs, job_count, total_blocks, per_lane, layout, in, out, follows, stream);
+        return launch_tring_hb5_w8(jobs, job_count, total_blocks, per_lane, layout, in, out, ahead, stream);
     if (half_bandwidth == 5 && window == 12)
-        return launch_tring_hb5_w12(jobs, job_count, total_blocks, per_lane, layout, in, out, follows, stream);
+        return launch_tring_hb5_w12(jobs, job_count, total_blocks, per_lane, layout, in, out, ahead, stream);
     if (half_bandwidth == 5 && window == 16)
-        return launch_tring_hb5_w16(jobs, job_count, total_blocks, per_lane, layout, in, out, follows, stream);
+        return launch_tring_hb5_w16(jobs, job_count, total_blocks, per_lane, layout, in, out, ahead, stream);
     if (half_bandwidth == 7 && window == 12)
-        return launch_tring_hb7_w12(jobs, job_count, total_blocks, per_lane, layout, in, out, follows, stream);
+        return launch_tring_hb7_w12(jobs, job_count, total_blocks, per_lane, layout, in, out, ahead, stream);
     if (half_bandwidth == 7 && window == 16)
-        return launch_tring_hb7_w16(jobs, job_count, total_blocks, per_lane, layout, in, out, follows, stream);
+        return launch_tring_hb7_w16(jobs, job_count, total_blocks, per_lane, layout, in, out, ahead, stream);
     return static_cast<int>(cudaErrorInvalidValue);
 }
 
-int launch_xring_hb1_w4(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb1_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb1_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb3_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb3_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb3_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb5_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb5_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb5_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb7_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb7_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb9_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
-int launch_xring_hb11_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, bool, void *);
+int launch_xring_hb1_w4(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb1_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb1_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb3_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb3_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb3_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb5_w8(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb5_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb5_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb7_w12(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb7_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb9_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
+int launch_xring_hb11_w16(const dev::StreamJob *, int, int, int, bool, dev::Sample, dev::Sample, RingAhead, void *);
 
 int launch_xring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
-                 int per_lane, bool tiled, dev::Sample in, dev::Sample out, bool follows, void *stream) {
+                 int per_lane, bool tiled, dev::Sample in, dev::Sample out, RingAhead ahead, void *stream) {
     if (half_bandwidth == 1 && window == 4)
-        return launch_xring_hb1_w4(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb1_w4(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 1 && window == 8)
-        return launch_xring_hb1_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb1_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 1 && window == 16)
-        return launch_xring_hb1_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb1_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 3 && window == 8)
-        return launch_xring_hb3_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb3_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 3 && window == 12)
-        return launch_xring_hb3_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb3_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 3 && window == 16)
-        return launch_xring_hb3_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb3_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 5 && window == 8)
-        return launch_xring_hb5_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb5_w8(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 5 && window == 12)
-        return launch_xring_hb5_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb5_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 5 && window == 16)
-        return launch_xring_hb5_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb5_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 7 && window == 12)
-        return launch_xring_hb7_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb7_w12(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 7 && window == 16)
-        return launch_xring_hb7_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb7_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 9 && window == 16)
-        return launch_xring_hb9_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb9_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     if (half_bandwidth == 11 && window == 16)
-        return launch_xring_hb11_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, follows, stream);
+        return launch_xring_hb11_w16(jobs, job_count, total_blocks, per_lane, tiled, in, out, ahead, stream);
     return static_cast<int>(cudaErrorInvalidValue);
 }
 

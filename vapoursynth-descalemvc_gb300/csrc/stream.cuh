@@ -102,12 +102,18 @@ constexpr int kTRingPitch = 34;
 // the vectors adjacent, that output (Float32) in tiles of 32 vectors, a
 // Float32 plane's rows in and out, or its columns.
 enum class RingLayout : std::int32_t { plain, tiled, rows, columns };
+// What a launch of these finds ahead of it on its stream.  ended: it starts once
+// that has ended.  own, any: it may start before (programmatic serialization); it
+// reads its jobs and records, and waits before it reads a sample.  own: a launch of
+// the same pass or the pass before, whose CTAs hold their tensor memory before
+// they let another start.  any: whatever the caller put there.  A CTA then allocates
+// its own tensor memory only after that wait: held before it, it could keep a grid ahead
+// that lets its dependents start before it allocates from ever ending.
+enum class RingAhead : std::int32_t { ended, own, any };
 // Chunk-delayed passes, the sample ring in tensor memory (tring_impl.cuh).
 // Every job of a launch has the same window (StreamPack::ring_window) and its
 // plan view the matching records; `per_lane` vectors a lane (1 or 2), CTAs of
-// kTRingThreads threads.  `follows`: the launch may start before the one ahead
-// of it on the stream has ended; it reads its jobs and records before it waits
-// for that one's results.
+// kTRingThreads threads.
 constexpr int kTStreamThreads = 128;   // default CTA size of the two-pass kernels
 // Float64 two-pass kernels: two warps a CTA spread a launch's segments more
 // evenly over the SMs, whose FP64 units bind (4K Spline64 frames on one
@@ -118,7 +124,7 @@ constexpr int kTRingThreads = 128;
 constexpr int kTResidentWarps = 16;    // resident warps per SM (128 registers a thread)
 constexpr int kMinSegmentChunks = 1;   // shortest segment, in chunks (StreamJob)
 int launch_tring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
-                 int per_lane, RingLayout layout, dev::Sample in, dev::Sample out, bool follows, void *stream);
+                 int per_lane, RingLayout layout, dev::Sample in, dev::Sample out, RingAhead ahead, void *stream);
 
 // Columns passes with fused candidate scoring (tscore_impl.cuh): as
 // the transposing passes, for Float32 intermediates with chunk-delayed records
@@ -134,7 +140,7 @@ int launch_tscore(const dev::StreamJob *jobs, int job_count, int total_blocks, i
 // of launch_tring; launch_tsolve (tsolve_impl.cuh) serves the plans whose
 // group refill exceeds that ring.
 int launch_xring(const dev::StreamJob *jobs, int job_count, int total_blocks, int half_bandwidth, int window,
-                 int per_lane, bool tiled, dev::Sample in, dev::Sample out, bool follows, void *stream);
+                 int per_lane, bool tiled, dev::Sample in, dev::Sample out, RingAhead ahead, void *stream);
 bool tsolve_supports(int half_bandwidth);
 int launch_tsolve(const dev::StreamJob *jobs, int job_count, int total_blocks, int threads, int half_bandwidth,
                   dev::Sample in, dev::Sample out, int record_floats, void *stream);

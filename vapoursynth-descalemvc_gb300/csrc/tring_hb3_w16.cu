@@ -5,9 +5,9 @@
 namespace dsmvc_gb {
 
 int launch_tring_hb3_w16(const dev::StreamJob *jobs, int count, int blocks, int per_lane, RingLayout layout,
-                       dev::Sample in, dev::Sample out, bool follows, void *stream) {
-    return per_lane == 2 ? rlaunch<3, 16, 2>(jobs, count, blocks, in, out, layout, follows, stream)
-                         : rlaunch<3, 16, 1>(jobs, count, blocks, in, out, layout, follows, stream);
+                       dev::Sample in, dev::Sample out, RingAhead ahead, void *stream) {
+    return per_lane == 2 ? rlaunch<3, 16, 2>(jobs, count, blocks, in, out, layout, ahead, stream)
+                         : rlaunch<3, 16, 1>(jobs, count, blocks, in, out, layout, ahead, stream);
 }
 
 } // namespace dsmvc_gb

@@ -142,14 +142,13 @@ struct RingFeeder {
 
     // `stage_at`, `mbar_at`: the warp's staging buffers and their barriers.
     __device__ __forceinline__ void init(const StreamJob &j, int samples, int first_vector, int count_vectors, int l,
-                                         unsigned ring_at, unsigned stage_at, unsigned mbar_at) {
+                                         unsigned stage_at, unsigned mbar_at) {
         job = &j;
         map = j.mapped ? reinterpret_cast<std::uint64_t>(j.map) : 0;
         first = first_vector;
         vectors = count_vectors;
         size = limit = samples;
         lane = l;
-        ring = ring_at;
         stage = stage_at;
         mbar = mbar_at;
         // Lanes past the warp's last vector repeat it: same samples, same
@@ -326,7 +325,8 @@ struct RingFeeder {
     }
 
     // `from`: a multiple of 16 at most the first window start.
-    __device__ __forceinline__ void start(int from) {
+    __device__ __forceinline__ void start(int from, unsigned ring_at) {
+        ring = ring_at;
         const float zero[8] = {};
         for (int c = 0; c < V * VC; c += 8) tm_st8(ring + c, zero);
         tm_wait_st();
@@ -591,16 +591,33 @@ __device__ __forceinline__ void rstore_wait() {
 }
 
 // Waits for the launch before this one, its results included, where this one
-// may start early (launch_tring's `follows`).  Every thread does: a launch is
+// may start early (RingAhead own, any).  Every thread does: a launch is
 // complete only after those before it.
 __device__ __forceinline__ void ring_launch_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
-// Lets such a launch behind this one start once every CTA is past this point.
+// Lets such a launch behind this one start once every CTA is past this point (and
+// holds its tensor memory).
 __device__ __forceinline__ void ring_launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
+// A CTA's tensor memory, by its first warp; *base after the next barrier.  Those
+// that an allocation waits for wait for nothing: they are past ring_launch_wait, or
+// wait behind launches that all hold theirs (RingAhead).
+template <int COLUMNS> __device__ __forceinline__ void ring_allocate(unsigned *base, int warp) {
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
+                     :: "r"(static_cast<unsigned>(__cvta_generic_to_shared(base))), "n"(COLUMNS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+    }
+}
+__device__ __forceinline__ void ring_allocated() {
+    asm volatile("tcgen05.fence::before_thread_sync;\n");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n");
+}
 
 template <int HB, int W, int V, RingLayout LAYOUT, class In, class Out>
 __global__ void __launch_bounds__(kRingThreads, 4 / V)
-tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
+tring_kernel(const StreamJob *__restrict__ jobs, int job_count, bool late) {
     using R = RingRecord<HB, W>;
     using Feed = RingFeeder<In, V, W, LAYOUT>;
     constexpr bool TILED = LAYOUT == RingLayout::tiled, ROWS = LAYOUT == RingLayout::rows;
@@ -641,35 +658,30 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
     if (c0 + 1 <= ce) tstage(bufs + ((c0 + 1) % 3) * R::CHUNK, p, c0 + 1, tid, kRingThreads);
     tcp_commit();
 
-    if (warp == 0) {
-        // The allocation ends: a CTA waiting for it holds none, and those that
-        // hold theirs wait for nothing of another CTA's.
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
-                     :: "r"(static_cast<unsigned>(__cvta_generic_to_shared(&tm_base))), "n"(COLUMNS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
-    }
+    if (!late) ring_allocate<COLUMNS>(&tm_base, warp);
     if (lane < kRingBuffers) {
         const unsigned mb = static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][lane]));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" :: "r"(mb), "r"(ring_arrivals<LAYOUT>(job, lead)) : "memory");
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;\n");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n");
+    ring_allocated();
 
     // The warp's vectors; a warp past its job's last vector only takes part
     // in the CTA's record copies and barriers.
     const int warp_first = (cta_warp + warp - job.first_block) * 32 * V;
     const int left = job.vectors - warp_first;
     const bool idle = left <= 0;
-    const unsigned tm = tm_base;
     Feed feed;
     feed.init(job, p.source_size, idle ? 0 : warp_first, idle ? 1 : min(left, 32 * V), lane,
-              tm + (static_cast<unsigned>(warp * 32) << 16),
               static_cast<unsigned>(__cvta_generic_to_shared(ring_smem + warp * kRingBuffers * Feed::BUFFER)),
               static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][0])));
     ring_launch_wait();
-    if (!idle) feed.start(c0 > 0 ? lead.first_sample : 0);
+    if (late) {
+        ring_allocate<COLUMNS>(&tm_base, warp);
+        ring_allocated();
+    }
+    const unsigned tm = tm_base;
+    if (!idle) feed.start(c0 > 0 ? lead.first_sample : 0, tm + (static_cast<unsigned>(warp * 32) << 16));
     ring_launch_next();
 
     Out *out[V];
@@ -748,12 +760,18 @@ tring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" :: "r"(tm), "n"(COLUMNS));
 }
 
-// Launches behind the launch before it on the stream or, `follows`, while that
-// one still ends: the way to the first sample (job table, records, tensor
+// Launches behind the launch before it on the stream or, unless that has `ended`,
+// while it still ends: the way to the first sample (job table, records, tensor
 // memory, barriers), up to 3 us of a pass, then runs beside it.  The kernels
-// read only what that launch does not write until ring_launch_wait.
-inline cudaError_t ring_launch(void (*kernel)(const StreamJob *, int), const StreamJob *jobs, int count, int blocks,
-                               int smem, bool follows, cudaStream_t s) {
+// read only what that launch does not write until ring_launch_wait.  Late
+// allocations (RingAhead any) keep some of it back: on the runs measured an SM took no
+// second such CTA before the first had allocated.  One Float32 bicubic frame on one
+// GB300, frames behind one another, us with each first launch behind the end of the
+// frame before, with late and with early allocations: 640x360 20.5, 16.2 and 15.9,
+// 1080p 26.7, 23.4 and 20.2, 4K 41.0, 36.4 and 35.5; eight 1080p planes' rows 41.0,
+// 35.2 and 33.8.
+inline cudaError_t ring_launch(void (*kernel)(const StreamJob *, int, bool), const StreamJob *jobs, int count, int blocks,
+                               int smem, RingAhead ahead, cudaStream_t s) {
     cudaLaunchAttribute early{};
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;
@@ -763,47 +781,47 @@ inline cudaError_t ring_launch(void (*kernel)(const StreamJob *, int), const Str
     config.dynamicSmemBytes = static_cast<std::size_t>(smem);
     config.stream = s;
     config.attrs = &early;
-    config.numAttrs = follows ? 1 : 0;
-    return cudaLaunchKernelEx(&config, kernel, jobs, count);
+    config.numAttrs = ahead == RingAhead::ended ? 0 : 1;
+    return cudaLaunchKernelEx(&config, kernel, jobs, count, ahead == RingAhead::any);
 }
 
 template <int HB, int W, int V, RingLayout LAYOUT, class In, class Out>
-int rlaunch_typed(const StreamJob *jobs, int count, int blocks, bool follows, cudaStream_t s) {
+int rlaunch_typed(const StreamJob *jobs, int count, int blocks, RingAhead ahead, cudaStream_t s) {
     constexpr int smem = 1024 + 3 * RingRecord<HB, W>::CHUNK * 4
         + kRingThreads / 32 * (kRingBuffers * RingFeeder<In, V, W, LAYOUT>::BUFFER
                                + (LAYOUT == RingLayout::rows ? V * 4096 : 0));
     auto kernel = tring_kernel<HB, W, V, LAYOUT, In, Out>;
     static SmemLimit limit;
     if (const cudaError_t e = limit.ensure(kernel, smem); e != cudaSuccess) return static_cast<int>(e);
-    return static_cast<int>(ring_launch(kernel, jobs, count, blocks, smem, follows, s));
+    return static_cast<int>(ring_launch(kernel, jobs, count, blocks, smem, ahead, s));
 }
 
 template <int HB, int W, int V>
 int rlaunch(const StreamJob *jobs, int count, int blocks, dev::Sample in, dev::Sample out, RingLayout layout,
-            bool follows, void *stream) {
+            RingAhead ahead, void *stream) {
     using dev::Sample;
     using std::uint16_t, std::uint8_t;
     using L = RingLayout;
     const auto s = static_cast<cudaStream_t>(stream);
     if (in == Sample::f32 && out == Sample::f32) {
         switch (layout) {
-        case L::plain: return rlaunch_typed<HB, W, V, L::plain, float, float>(jobs, count, blocks, follows, s);
-        case L::tiled: return rlaunch_typed<HB, W, V, L::tiled, float, float>(jobs, count, blocks, follows, s);
-        case L::rows: return rlaunch_typed<HB, W, V, L::rows, float, float>(jobs, count, blocks, follows, s);
-        case L::columns: return rlaunch_typed<HB, W, V, L::columns, float, float>(jobs, count, blocks, follows, s);
+        case L::plain: return rlaunch_typed<HB, W, V, L::plain, float, float>(jobs, count, blocks, ahead, s);
+        case L::tiled: return rlaunch_typed<HB, W, V, L::tiled, float, float>(jobs, count, blocks, ahead, s);
+        case L::rows: return rlaunch_typed<HB, W, V, L::rows, float, float>(jobs, count, blocks, ahead, s);
+        case L::columns: return rlaunch_typed<HB, W, V, L::columns, float, float>(jobs, count, blocks, ahead, s);
         }
     }
     if (out == Sample::f32 && layout == L::tiled) {
-        if (in == Sample::u16) return rlaunch_typed<HB, W, V, L::tiled, uint16_t, float>(jobs, count, blocks, follows, s);
-        if (in == Sample::u8) return rlaunch_typed<HB, W, V, L::tiled, uint8_t, float>(jobs, count, blocks, follows, s);
+        if (in == Sample::u16) return rlaunch_typed<HB, W, V, L::tiled, uint16_t, float>(jobs, count, blocks, ahead, s);
+        if (in == Sample::u8) return rlaunch_typed<HB, W, V, L::tiled, uint8_t, float>(jobs, count, blocks, ahead, s);
     }
     if (out == Sample::f32 && layout == L::plain) {
-        if (in == Sample::u16) return rlaunch_typed<HB, W, V, L::plain, uint16_t, float>(jobs, count, blocks, follows, s);
-        if (in == Sample::u8) return rlaunch_typed<HB, W, V, L::plain, uint8_t, float>(jobs, count, blocks, follows, s);
+        if (in == Sample::u16) return rlaunch_typed<HB, W, V, L::plain, uint16_t, float>(jobs, count, blocks, ahead, s);
+        if (in == Sample::u8) return rlaunch_typed<HB, W, V, L::plain, uint8_t, float>(jobs, count, blocks, ahead, s);
     }
     if (in == Sample::f32 && layout == L::plain) {
-        if (out == Sample::u16) return rlaunch_typed<HB, W, V, L::plain, float, uint16_t>(jobs, count, blocks, follows, s);
-        if (out == Sample::u8) return rlaunch_typed<HB, W, V, L::plain, float, uint8_t>(jobs, count, blocks, follows, s);
+        if (out == Sample::u16) return rlaunch_typed<HB, W, V, L::plain, float, uint16_t>(jobs, count, blocks, ahead, s);
+        if (out == Sample::u8) return rlaunch_typed<HB, W, V, L::plain, float, uint8_t>(jobs, count, blocks, ahead, s);
     }
     return static_cast<int>(cudaErrorInvalidValue);
 }

@@ -5,9 +5,9 @@
 namespace dsmvc_gb {
 
 int launch_xring_hb7_w16(const dev::StreamJob *jobs, int count, int blocks, int per_lane, bool tiled,
-                       dev::Sample in, dev::Sample out, bool follows, void *stream) {
-    return per_lane == 2 ? xrlaunch<7, 16, 2>(jobs, count, blocks, in, out, tiled, follows, stream)
-                         : xrlaunch<7, 16, 1>(jobs, count, blocks, in, out, tiled, follows, stream);
+                       dev::Sample in, dev::Sample out, RingAhead ahead, void *stream) {
+    return per_lane == 2 ? xrlaunch<7, 16, 2>(jobs, count, blocks, in, out, tiled, ahead, stream)
+                         : xrlaunch<7, 16, 1>(jobs, count, blocks, in, out, tiled, ahead, stream);
 }
 
 } // namespace dsmvc_gb

@@ -38,7 +38,7 @@ __device__ __forceinline__ void xstage(float *buf, const float *from, int floats
 
 template <int HB, int W, int V, bool TILED, class In, class Out>
 __global__ void __launch_bounds__(kRingThreads, V == 1 ? 4 : 3)
-xring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
+xring_kernel(const StreamJob *__restrict__ jobs, int job_count, bool late) {
     using R = RingRecord<HB, W>;
     using Feed = RingFeeder<In, V, W, RingLayout::plain>;
     constexpr int LC = kTChunk, WARPS = kRingThreads / 32, G = 8;
@@ -73,31 +73,28 @@ xring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
     if (fc0 + 1 <= fce)
         xstage(bufs + ((fc0 + 1) % 3) * FORWARD, p.forward + static_cast<std::int64_t>(fc0 + 1) * FORWARD, FORWARD, tid);
     tcp_commit();
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
-                     :: "r"(static_cast<unsigned>(__cvta_generic_to_shared(&tm_base))), "n"(COLUMNS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
-    }
+    if (!late) ring_allocate<COLUMNS>(&tm_base, warp);
     if (lane < kRingBuffers) {
         const unsigned mb = static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][lane]));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" :: "r"(mb), "r"(ring_arrivals<RingLayout::plain>(job, lead)) : "memory");
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;\n");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n");
+    ring_allocated();
 
     const int warp_first = (cta_warp + warp - job.first_block) * 32 * V;
     const int left = job.vectors - warp_first;
     const bool idle = left <= 0;
-    const unsigned tm = tm_base;
     Feed feed;
     feed.init(job, p.source_size, idle ? 0 : warp_first, idle ? 1 : min(left, 32 * V), lane,
-              tm + (static_cast<unsigned>(warp * 32) << 16),
               static_cast<unsigned>(__cvta_generic_to_shared(ring_smem + warp * kRingBuffers * Feed::BUFFER)),
               static_cast<unsigned>(__cvta_generic_to_shared(&feed_bar[warp][0])));
     ring_launch_wait();
-    if (!idle) feed.start(fc0 > 0 ? lead.first_sample : 0);
+    if (late) {
+        ring_allocate<COLUMNS>(&tm_base, warp);
+        ring_allocated();
+    }
+    const unsigned tm = tm_base;
+    if (!idle) feed.start(fc0 > 0 ? lead.first_sample : 0, tm + (static_cast<unsigned>(warp * 32) << 16));
     ring_launch_next();
 
     // Forward value of destination j at yp[a][j * y_elem].  Lanes past the
@@ -233,37 +230,37 @@ xring_kernel(const StreamJob *__restrict__ jobs, int job_count) {
 }
 
 template <int HB, int W, int V, bool TILED, class In, class Out>
-int xrlaunch_typed(const StreamJob *jobs, int count, int blocks, bool follows, cudaStream_t s) {
+int xrlaunch_typed(const StreamJob *jobs, int count, int blocks, RingAhead ahead, cudaStream_t s) {
     using R = RingRecord<HB, W>;
     constexpr int smem = 1024 + 3 * R::GROUPS * R::GROUP * 4
         + kRingThreads / 32 * kRingBuffers * RingFeeder<In, V, W, RingLayout::plain>::BUFFER;
     auto kernel = xring_kernel<HB, W, V, TILED, In, Out>;
     static SmemLimit limit;
     if (const cudaError_t e = limit.ensure(kernel, smem); e != cudaSuccess) return static_cast<int>(e);
-    return static_cast<int>(ring_launch(kernel, jobs, count, blocks, smem, follows, s));
+    return static_cast<int>(ring_launch(kernel, jobs, count, blocks, smem, ahead, s));
 }
 
 template <int HB, int W, int V>
 int xrlaunch(const StreamJob *jobs, int count, int blocks, dev::Sample in, dev::Sample out, bool tiled,
-             bool follows, void *stream) {
+             RingAhead ahead, void *stream) {
     using dev::Sample;
     using std::uint16_t, std::uint8_t;
     const auto s = static_cast<cudaStream_t>(stream);
     if (out == Sample::f32) {
         if (in == Sample::f32)
-            return tiled ? xrlaunch_typed<HB, W, V, true, float, float>(jobs, count, blocks, follows, s)
-                         : xrlaunch_typed<HB, W, V, false, float, float>(jobs, count, blocks, follows, s);
+            return tiled ? xrlaunch_typed<HB, W, V, true, float, float>(jobs, count, blocks, ahead, s)
+                         : xrlaunch_typed<HB, W, V, false, float, float>(jobs, count, blocks, ahead, s);
         if (in == Sample::u16)
-            return tiled ? xrlaunch_typed<HB, W, V, true, uint16_t, float>(jobs, count, blocks, follows, s)
-                         : xrlaunch_typed<HB, W, V, false, uint16_t, float>(jobs, count, blocks, follows, s);
+            return tiled ? xrlaunch_typed<HB, W, V, true, uint16_t, float>(jobs, count, blocks, ahead, s)
+                         : xrlaunch_typed<HB, W, V, false, uint16_t, float>(jobs, count, blocks, ahead, s);
         if (in == Sample::u8)
-            return tiled ? xrlaunch_typed<HB, W, V, true, uint8_t, float>(jobs, count, blocks, follows, s)
-                         : xrlaunch_typed<HB, W, V, false, uint8_t, float>(jobs, count, blocks, follows, s);
+            return tiled ? xrlaunch_typed<HB, W, V, true, uint8_t, float>(jobs, count, blocks, ahead, s)
+                         : xrlaunch_typed<HB, W, V, false, uint8_t, float>(jobs, count, blocks, ahead, s);
     }
     if (in == Sample::f32 && out == Sample::u16)
-        return xrlaunch_typed<HB, W, V, false, float, uint16_t>(jobs, count, blocks, follows, s);
+        return xrlaunch_typed<HB, W, V, false, float, uint16_t>(jobs, count, blocks, ahead, s);
     if (in == Sample::f32 && out == Sample::u8)
-        return xrlaunch_typed<HB, W, V, false, float, uint8_t>(jobs, count, blocks, follows, s);
+        return xrlaunch_typed<HB, W, V, false, float, uint8_t>(jobs, count, blocks, ahead, s);
     return static_cast<int>(cudaErrorInvalidValue);
 }
 
