@@ -571,8 +571,8 @@ struct Executor::Impl {
     // DSMVC_GB_STREAM=0 keeps every plan on the sequential kernels (the
     // counterpart of the reference's DSMVC_GPU_SOLVE_PARTITION switch).
     bool allow_stream = true;
-    // DSMVC_GB_PAIRED=1 runs every chunk-delayed 2D pass with two vectors a
-    // lane, in whole vectors (kind 4).
+    // DSMVC_GB_PAIRED=1 runs every pass with the ring in tensor memory with two
+    // vectors a lane, the chunk-delayed 2D passes in whole vectors (kind 4).
     bool allow_paired = false;
     // DSMVC_GB_EXACT=1 runs every admitted 2D pass on the two-pass
     // transposing kernels; otherwise they serve the plans the chunk-delayed
@@ -926,7 +926,9 @@ std::vector<Item> segment_items(const std::vector<Item> &items, int vectors_per_
 void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                              const std::function<char *(std::size_t)> &scratch, std::uint32_t *status,
                              const Tuning *tuning, int vectors_per_warp) {
-    if (!vectors_per_warp && allow_paired) vectors_per_warp = 64;
+    // Vectors a lane of the launches with the ring in tensor memory; 0: by launch.
+    const bool paired = !vectors_per_warp && allow_paired;
+    const int forced_lanes = paired ? 2 : vectors_per_warp / 32;
     auto &temporaries = out.temporaries;
     // Per task: which kernels run each pass, and the scratch they need.
     struct Route {
@@ -991,7 +993,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
                 if (!allow_stream) return 0;
                 const bool delayed = dp.stream_t && dp.ring_window;
                 if (dp.stream_x && (prefer_exact || !delayed)) return 5;
-                if (delayed) return vectors_per_warp == 64 ? 4 : 3;
+                if (delayed) return paired ? 4 : 3;
                 return 0;
             };
             r.h_kind = pass_kind(*r.h);
@@ -1389,7 +1391,7 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
         } else if (ring) {
             // The split does not depend on the vectors a lane: neither do the
             // results.
-            const std::size_t whole = items.size();
+            const std::size_t jobs = items.size();
             const bool floats = key.in == dev::Sample::f32 && key.out == dev::Sample::f32;
             if (key.kind == 3)
                 items = segment_items(items, 32, segment_mode, warp_slots, 1, kMinSegmentChunks, floats && key.hb > 1);
@@ -1400,12 +1402,12 @@ void Executor::Impl::compile(const std::vector<PlaneTask> &tasks, Compiled &out,
             const long sms = warp_slots / kTResidentWarps;
             bool pair = warps >= kPairingWarps * sms;
             if (key.kind == 3) {
-                const bool ranges = items.size() > whole;
+                const bool ranges = items.size() > jobs;
                 pair = pair && key.hb > 1
                     && !(ranges && (warps < kPairingRanges * sms
                                     || (warp_slots / 8 < run_ctas(items, 64) && run_ctas(items, 32) <= warp_slots / 4)));
             }
-            if (!vectors_per_warp && pair) per_lane = 2;
+            per_lane = forced_lanes ? forced_lanes : pair ? 2 : 1;
         }
         if (ring)
             for (auto &it : items) {
@@ -2264,6 +2266,7 @@ std::vector<BatchGroup> PreparedBatch::groups() const {
         g.threads = l.threads;
         g.blocks = l.blocks;
         g.jobs = l.count;
+        g.per_lane = ring_kind(l.kind) || (l.kind == 5 && l.variant) ? l.per_lane : 0;
         g.name = kernel_name({l.pass, l.kind, l.hb, l.in, l.out, l.variant});
         out.push_back(g);
     }

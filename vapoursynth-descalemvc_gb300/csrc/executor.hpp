@@ -112,6 +112,7 @@ struct BatchGroup {
     int threads = 0;      // CTA size
     int blocks = 0;
     int jobs = 0;
+    int per_lane = 0;     // vectors a lane of launches with the ring in tensor memory, else 0
     std::string name;
 };
 
@@ -205,10 +206,11 @@ public:
     // `scratch` the batch's intermediate planes live in that caller-owned
     // device buffer of `scratch_capacity` bytes (batches launched one after
     // another may share it); otherwise the batch allocates its own.
-    // `vectors_per_warp` picks the transposing Float32 kernels' right-hand
-    // sides per warp: 32 (one vector a lane), 64 (two a lane, the paired
-    // kernels, where a plan admits them; same results bit for bit), or 0
-    // for the executor's default (DSMVC_GB_PAIRED).  `parts`: 1 launches
+    // `vectors_per_warp` picks the right-hand sides per warp of the Float32
+    // launches with the ring in tensor memory: 32 (one vector a lane), 64 (two a
+    // lane), or 0, each launch by its size.  The results are the same bits.
+    // (DSMVC_GB_PAIRED=1 makes 0 two a lane in all of them, the chunk-delayed 2D
+    // passes in whole vectors.)  `parts`: 1 launches
     // every task in one sequence of kernels; 2 splits the tasks where the
     // source pixels are halved and launches the halves on the caller's
     // stream and a second one forked from it and joined back, so that one

@@ -204,7 +204,7 @@ struct Sweep::Impl {
     std::map<const AxisPlan *, std::array<unsigned, 2>> windows;   // walk_windows: horizontal, vertical
     int segment_rows = 32;
     int best_segment = 32;
-    int vectors_per_warp = 0;   // 0: the executor's default; 32 / 64 once tuned
+    int vectors_per_warp = 0;   // PreparedBatch's: 0 by launch, 32 or 64 where tuning found them faster
     BatchTuning tuning;
     double tune_ms = 0.0;
     cudaGraph_t graph = nullptr;
@@ -650,37 +650,43 @@ struct Sweep::Impl {
         return ms / static_cast<float>(reps);
     }
 
-    // Times the first wave's descale with one and with two right-hand sides
-    // a lane (32 or 64 vectors a warp), then every launch group of it at
-    // each candidate CTA size, and the scoring column pass at each row
+    // Times the first wave's descale with the vectors a lane that each launch's
+    // size gives it and, where that mixes one and two or two may be faster, with
+    // one and with two in all of them, then every launch group of it at each
+    // candidate CTA size, and the scoring column pass at each row
     // segment (unfused candidates); keeps the fastest of each.  Scores do
     // not depend on the choices: every kernel variant gives each output bit
     // for bit, and the fused scoring kernel has one launch shape.
     void autotune() {
         const auto t0 = std::chrono::steady_clock::now();
         Wave &w = waves.front();
-        // Two right-hand sides a lane only where some plan runs the
-        // chunk-delayed kernels: otherwise both batches are the same launches.
-        auto single = executor->prepare_batch(w.tasks, nullptr, scratch_mem.data(), scratch_capacity, 32);
-        auto paired = executor->prepare_batch(w.tasks, nullptr, scratch_mem.data(), scratch_capacity, 64);
-        const auto paired_groups = paired->groups();
-        vectors_per_warp = 32;
-        if (std::any_of(paired_groups.begin(), paired_groups.end(), [](const BatchGroup &g) { return g.kind == 4; })) {
-            const float ms32 = time_ms([&] { single->launch(stream); }, 2);
-            const float ms64 = time_ms([&] { paired->launch(stream); }, 2);
+        auto chosen = executor->prepare_batch(w.tasks, nullptr, scratch_mem.data(), scratch_capacity, 0);
+        auto keys = chosen->groups();
+        auto runs = [&](int lanes) {
+            return std::any_of(keys.begin(), keys.end(), [&](const BatchGroup &g) { return g.per_lane == lanes; });
+        };
+        vectors_per_warp = 0;
+        const bool other[2] = {runs(2), runs(1)};   // where one, or two, in all of them differs
+        float fastest = other[0] || other[1] ? time_ms([&] { chosen->launch(stream); }, 2) : 0.0F;
+        for (const int lanes : {1, 2}) {
+            if (!other[lanes - 1]) continue;
+            auto batch = executor->prepare_batch(w.tasks, nullptr, scratch_mem.data(), scratch_capacity, 32 * lanes);
+            const float ms = time_ms([&] { batch->launch(stream); }, 2);
             check(cudaStreamSynchronize(stream), "synchronizing");
-            if (ms64 < ms32) vectors_per_warp = 64;
+            if (ms >= fastest) continue;
+            fastest = ms;
+            vectors_per_warp = 32 * lanes;
+            keys = batch->groups();
         }
+        check(cudaStreamSynchronize(stream), "synchronizing");
+        chosen.reset();
         std::map<std::array<int, 6>, std::pair<float, int>> best;
-        const auto keys = (vectors_per_warp == 64 ? paired : single)->groups();
-        single.reset();
-        paired.reset();
         // 32-thread CTAs never win on these kernels (one warp per record copy).
         for (const int threads : {64, 128, 256}) {
             BatchTuning all;
             for (const auto &g : keys) {
                 // The kernels with the ring in tensor memory have one CTA size.
-                const bool ring = g.kind == 3 || g.kind == 4 || (g.kind == 5 && g.key[5]);
+                const bool ring = g.per_lane > 0;
                 const int most = g.kind >= 3 && !ring ? 256 : 128;
                 if (g.kind != 2 && g.kind <= 6 && threads <= most && (!ring || threads == 128)) all[g.key] = threads;
             }
@@ -874,7 +880,9 @@ SweepInfo Sweep::info() const {
     i.fused_candidates = m.fused_count;
     i.tune_milliseconds = m.tune_ms;
     i.segment_rows = m.segment_rows;
-    i.vectors_per_warp = m.vectors_per_warp ? m.vectors_per_warp : 32;
+    i.vectors_per_warp = 32;
+    for (const auto &w : m.waves)
+        for (const auto &g : w.batch->groups()) i.vectors_per_warp = std::max(i.vectors_per_warp, 32 * g.per_lane);
     i.tuning = m.tuning;
     return i;
 }

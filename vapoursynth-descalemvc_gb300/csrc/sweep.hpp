@@ -50,7 +50,7 @@ struct SweepInfo {
     std::size_t kernel_launches = 0;  // per run()
     double tune_milliseconds = 0.0;
     int segment_rows = 0;
-    int vectors_per_warp = 32;        // chosen right-hand sides per warp (32 or 64)
+    int vectors_per_warp = 32;        // most right-hand sides per warp of a launch (32 or 64)
     int fused_candidates = 0;         // scored inside their columns pass
     BatchTuning tuning;               // chosen CTA sizes per launch group
 };
