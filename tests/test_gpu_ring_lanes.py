@@ -4,8 +4,10 @@ scores do not depend on what its tuning chose."""
 import numpy as np
 import pytest
 
+import oracle as O
 from conftest import _executor_with
 from test_gpu_launch_order import call, captured
+from test_gpu_ring import make_input, pair
 
 pytestmark = pytest.mark.gpu
 
@@ -71,3 +73,55 @@ def test_scores_do_not_depend_on_the_tuning(gb, executor):
         scores.append(sweep.scores(0))
         sweep.close()
     assert np.array_equal(*scores)
+
+
+@pytest.fixture(scope="module")
+def exact_two_a_lane(gb):
+    ex = _executor_with(gb, "DSMVC_GB_EXACT", "1", DSMVC_GB_SEGMENTS="1", DSMVC_GB_PAIRED="1")
+    yield ex
+    ex.close()
+
+
+# Half-bandwidths 3, 5, 9 and 11; vectors on either side of 64 a warp, 256 a CTA.
+@pytest.mark.parametrize("width,height", [(90, 33), (97, 64), (131, 129), (388, 257)])
+@pytest.mark.parametrize("kernel,taps,ratio", [("bicubic", 3, 1.5), ("lanczos", 3, 1.4), ("spline64", 3, 1.5),
+                                               ("lanczos", 5, 1.3), ("lanczos", 6, 1.2)])
+def test_two_pass_kernels(gb, exact_two_a_lane, kernel, taps, ratio, width, height):
+    """Two-pass kernels at two vectors a lane: the reference CUDA order bit for bit."""
+    h, v, oh, ov = pair(gb, kernel, taps, ratio, width, height)
+    for sample in ("f32", "u16", "u8"):
+        conv = gb.integer_conversion({"u16": 16, "u8": 8}[sample], False, False) if sample != "f32" else None
+        x = make_input(height, width, sample, 6)
+        want = O.inverse_2d_gpu_order(oh, ov, x, conv) if conv else O.inverse_2d_gpu_order(oh, ov, x)
+        assert np.array_equal(exact_two_a_lane.inverse_2d(h, v, x, conv), want), sample
+
+
+@pytest.mark.parametrize("pitch", [112, 97])
+@pytest.mark.parametrize("sample", ["f32", "u16", "u8"])
+def test_large_two_pass_batches(gb, whole_executor, sample, pitch):
+    """Enough planes in one part for two vectors a lane in both passes, rows that a tensor map
+    admits and rows that none does: the samples of batches at one."""
+    import torch
+    w, h, ow, oh = 97, 97, 65, 61
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    planes = -(-8 * sms // -(-ow // 32))
+    dtype = {"f32": torch.float32, "u16": torch.int16, "u8": torch.uint8}[sample]
+    code, size = {"f32": (0, 4), "u16": (2, 2), "u8": (1, 1)}[sample]
+    conv = gb.integer_conversion(8 * size, False, False) if code else None
+    hp, vp = (gb.AxisPlan(gb.AxisRequest(n, m, float(m), 0.0, "spline64", 3, 0.0, 0.5, 1.1, "symmetric", 0))
+              for n, m in ((w, ow), (h, oh)))
+    x = np.random.default_rng(size).random((planes, h, pitch), dtype=np.float32)
+    x = torch.from_numpy(x if not code else (x * ((1 << 8 * size) - 1)).astype(np.int64)).to(dtype).cuda()
+    outs = [torch.zeros((planes, oh, ow), dtype=dtype, device="cuda") for _ in range(2)]
+    task = lambda i, out: gb.PlaneTask(hp, vp, x[i].data_ptr(), pitch, out[i].data_ptr(), ow, code, 0, conv)
+    torch.cuda.synchronize()
+    for out, group, lanes in ((outs[0], planes, 2), (outs[1], 40, 1)):
+        for first in range(0, planes, group):
+            part = range(first, min(first + group, planes))
+            batch = whole_executor.prepare_batch([task(i, out) for i in part], parts=1)
+            if first == 0:
+                spare = torch.zeros(8, device="cuda")
+                assert grids(batch, spare) == [-(-len(part) * -(-n // (32 * lanes)) // 4) for n in (h, ow)]
+            batch.launch(0)
+            batch.check(0)
+    assert torch.equal(*outs)
