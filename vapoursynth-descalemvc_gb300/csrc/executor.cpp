@@ -2170,6 +2170,8 @@ struct PreparedBatch::Impl {
     };
     std::vector<std::unique_ptr<Branch>> branches;
     void launch_branches(cudaStream_t s);
+    // A launch's fork and join events are its own until it is enqueued.
+    std::mutex forking;
     std::uint32_t *status = nullptr;       // device
     std::uint32_t *status_host = nullptr;  // pinned
     ~Impl() {
@@ -2198,6 +2200,21 @@ PreparedBatch::~PreparedBatch() {
     cudaDeviceSynchronize();
     impl_.reset();
 }
+
+namespace {
+
+// Whether `side`, a stream of a batch, may fork from `s`: not while another stream's
+// capture holds it (from its join there until that capture ends).
+bool forkable(cudaStream_t s, cudaStream_t side) {
+    cudaStreamCaptureStatus status[2] = {cudaStreamCaptureStatusNone, cudaStreamCaptureStatusNone};
+    unsigned long long id[2] = {0, 0};
+    cuda_check(cudaStreamGetCaptureInfo(side, &status[1], &id[1]), "reading capture status");
+    if (status[1] == cudaStreamCaptureStatusNone) return true;
+    cuda_check(cudaStreamGetCaptureInfo(s, &status[0], &id[0]), "reading capture status");
+    return status[0] == status[1] && id[0] == id[1];
+}
+
+} // namespace
 
 // A pass's launches on the caller's stream and the branches, forked from it and
 // joined back (capturable); those with the fewest, longest vectors (the later
@@ -2230,12 +2247,17 @@ void PreparedBatch::launch(void *stream) {
     DeviceGuard guard(impl_->owner->device);
     auto s = static_cast<cudaStream_t>(stream);
     auto &m = *impl_;
-    if (!m.branches.empty() && !m.owner->profiling) {
+    std::scoped_lock lock(m.forking);
+    if (!m.branches.empty() && !m.owner->profiling && forkable(s, m.branches[0]->stream)) {
         m.launch_branches(s);
         return;
     }
     if (m.parts.size() == 1) {
         m.owner->launch(m.parts[0]->compiled, m.parts[0]->table.data(), s, m.status, true);
+        return;
+    }
+    if (!forkable(s, m.side)) {
+        for (const auto &part : m.parts) m.owner->launch(part->compiled, part->table.data(), s, m.status);
         return;
     }
     // Fork: the second part's stream waits for the caller's; join: the
