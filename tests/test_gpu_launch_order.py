@@ -72,3 +72,41 @@ def test_first_launch_allocates_late(gb, executor, kernel, taps, blur, axes):
     assert late[0] or not early[0]
     assert early[1:] == [True] * (len(own) - 1) and not any(late[1:])
     call("cuGraphDestroy", graph)
+
+
+@pytest.mark.parametrize("axes", ["both", "rows"])
+def test_input_of_another_stream(gb, whole_executor, axes):
+    """Input written on another stream, its event waited for behind the pass before: a first
+    launch that starts early still waits for it."""
+    import torch
+    w, h, ow, oh = 640, 360, 427, 240 if axes == "both" else 360
+    plan = lambda n, m: gb.AxisPlan(gb.AxisRequest(n, m, float(m), 0.0, "bicubic", 3, 0.0, 0.5, 1.0, "symmetric", 0))
+    hp, vp = plan(w, ow), plan(h, oh) if axes == "both" else None
+    frames = torch.from_numpy(np.random.default_rng(3).random((8, h, w), dtype=np.float32)).cuda()
+    x, y = torch.zeros((h, w), device="cuda"), torch.zeros((oh, ow), device="cuda")
+    batch = whole_executor.prepare_batch([gb.PlaneTask(hp, vp, x.data_ptr(), w, y.data_ptr(), ow, 0, 0 if vp else h)])
+    want, got = (torch.zeros((8, oh, ow), device="cuda") for _ in range(2))
+    load = torch.rand(1 << 24, device="cuda")
+    for k in range(8):
+        x.copy_(frames[k])
+        torch.cuda.synchronize()
+        batch.launch(0)
+        batch.check(0)
+        want[k].copy_(y)
+    torch.cuda.synchronize()
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    for _ in range(4):
+        got.zero_()
+        torch.cuda.synchronize()
+        for k in range(8):
+            with torch.cuda.stream(two):
+                two.wait_stream(one)
+                load.add_(0.0)
+                x.copy_(frames[k])
+            with torch.cuda.stream(one):
+                batch.launch(one.cuda_stream)            # the frame before, or this one: overwritten below
+                one.wait_stream(two)
+                batch.launch(one.cuda_stream)
+                got[k].copy_(y)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
