@@ -370,7 +370,12 @@ int dsmvc_gb_stream_release(dsmvc_gb_executor *executor, void *stream);
  * plane (src/cuda/cuda_launch.hpp:11-149).  dsmvc_gb_batch_launch issues
  * kernels only -- no copy, allocation or host synchronisation -- so it may
  * be captured into a CUDA graph; launches of one batch must be ordered (one
- * stream or a graph) because they share the batch's scratch.
+ * stream or a graph) because they share the batch's scratch.  The first
+ * kernel of a batch in one part may start before the kernel ahead of it on
+ * `stream` has ended and waits for that one before it reads or writes any
+ * plane: ordered behind all that is ahead, unless the caller launched that
+ * kernel with programmatic stream serialization and it does not wait for its
+ * own predecessor.  No other thread may enqueue on `stream` during the call.
  * dsmvc_gb_batch_check waits for `stream` and reports Float64 non-finite
  * data seen by any earlier launch.  The tasks' buffers, their plans and the
  * executor must outlive the batch. */
@@ -387,7 +392,9 @@ int dsmvc_gb_batch_info(const dsmvc_gb_batch *batch, int64_t *kernel_launches,
  * `stream` and on a stream of the batch forked from it and joined back to it
  * (stream-ordered, capturable), so that one half's second pass overlaps the
  * other's first; 0 (what dsmvc_gb_batch_create does) chooses 2 for 8 tasks
- * of two axes or more.  dsmvc_gb_batch_parts reports the count. */
+ * of two axes or more, but 1 for small batches of Float32 planes, whose
+ * vectors one part's segments spread over the GPU.  dsmvc_gb_batch_parts
+ * reports the count. */
 int dsmvc_gb_batch_create_parts(dsmvc_gb_executor *executor,
                                 const dsmvc_gb_plane_task *tasks, int32_t count,
                                 int32_t parts, dsmvc_gb_batch **out);

@@ -215,8 +215,8 @@ public:
     // source pixels are halved and launches the halves on the caller's
     // stream and a second one forked from it and joined back, so that one
     // half's second pass overlaps the other's first (measured 14 % faster on
-    // 32 4K planes); 0 chooses 2 for batches of 8 tasks or more that own
-    // their scratch.  Results do not depend on the parts beyond what
+    // 32 4K planes); 0 chooses 2 for batches of 8 tasks of two axes or more that
+    // own their scratch, but 1 for small batches of Float32 planes.  Results do not depend on the parts beyond what
     // segment splits already allow (DSMVC_GB_SEGMENTS=1: none).
     [[nodiscard]] std::unique_ptr<PreparedBatch> prepare_batch(const std::vector<PlaneTask> &tasks,
                                                              const BatchTuning *tuning = nullptr,

@@ -643,7 +643,8 @@ class Executor:
     def prepare_batch(self, tasks: Sequence[PlaneTask], parts: int = 0) -> "PreparedBatch":
         """Routes and uploads `tasks` once; PreparedBatch.launch() then
         issues only the kernels (capturable into a CUDA graph).  `parts`: 1
-        or 2 (overlapping halves on two streams), 0 = 2 for 8 tasks or more."""
+        or 2 (overlapping halves on two streams); 0 = 2 for 8 tasks of two axes
+        or more, but 1 for small batches of Float32 planes."""
         return PreparedBatch(self, tasks, parts)
 
     def stream_check(self, stream: int = 0) -> None:
