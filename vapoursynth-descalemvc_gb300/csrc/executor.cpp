@@ -587,8 +587,9 @@ struct Executor::Impl {
     // kernels add one residual refinement step per pass (refine64.cu): the
     // columns pass then writes a Float64 plane, refined and converted last.
     bool f64_refine = false;
-    // Default CTA size of the transposing kernels (DSMVC_GB_TSTREAM_THREADS,
-    // 32..256 in multiples of 32); batches may tune it per launch group.
+    // Default CTA sizes of the two-pass kernels without the ring in tensor memory
+    // (DSMVC_GB_TSTREAM_THREADS, 32..256 in multiples of 32); batches may tune them
+    // per launch group.
     int tstream_threads = kTStreamThreads;
     int tsolve64_threads = kTSolve64Threads;
     // Segments of the chunk-delayed transposing passes (DSMVC_GB_SEGMENTS):
@@ -740,7 +741,8 @@ struct GroupKey {
                      // fused sweep scoring
     int hb;
     dev::Sample in, out;
-    int variant = 0; // kind 3: the kernels' window (8, or 12 / 16 for grouped records), else 0
+    int variant = 0; // kinds 3, 4, 5, 10: the compiled window, 0 without the ring in tensor
+                     // memory, and kTiled; kind 9: the records' window
     bool operator<(const GroupKey &o) const {
         return std::tie(pass, kind, hb, in, out, variant)
             < std::tie(o.pass, o.kind, o.hb, o.in, o.out, o.variant);
@@ -777,9 +779,10 @@ int compiled_window(const DevicePlan &dp) { return dp.ring_window; }
 // 1080p 17.3 and 18.2, twelve 61 and 79, one of 4K 32 and 40, 32 of 4K 490 and 574.
 constexpr int kPairingWarps = 8, kPairingRanges = 10;
 
-// One-axis passes in segments: two chunks of zero-history warm-up leave below
-// 2^-52 of it, so that a segment's forward values come to the whole vector's
-// own bits.  Ranges of at least three chunks (two cost two 1080p planes 2 us of
+// One-axis passes in segments: two chunks of zero-history warm-up, each of which
+// leaves below 2^-26 a slot, leave below half-bandwidth x 2^-52 of a history in each.
+// On every vector tried (test_one_axis, test_gpu_ring.py) a segment's values were
+// then the whole vector's bits; nothing guarantees it.  Ranges of at least three chunks (two cost two 1080p planes 2 us of
 // 25 in repeated work; four cost one plane 2 of 21 in latency).
 constexpr int kAxisMargin = 2, kAxisMinChunks = 3;
 
@@ -802,6 +805,8 @@ int Executor::Impl::fused_window(const DevicePlan &dp) const {
 
 namespace {
 
+// Labels that callers read (kernel_times): a kind keeps its own whatever kernel
+// serves it.
 std::string kernel_name(const GroupKey &k) {
     static const char *kinds[] = {"axis_f32", "axis_f64", "stream_f32", "tstream_f32", "tstream2_f32",
                                   "tsolve_f32", "tsolve_f64", "refine_f64", "convert_f64", "tscore_f32",
@@ -2327,7 +2332,7 @@ std::size_t PreparedBatch::parts() const { return impl_->parts.size(); }
 
 std::size_t Executor::batch_scratch_bound(const std::vector<PlaneTask> &tasks) {
     // Per task: the intermediate plane (destinations of the first pass x
-    // sources of the second, rows padded to 4) plus a forward plane of the
+    // sources of the second, rows padded to 4, or to tiles of 32) plus a forward plane of the
     // output's size, in the route's sample width; 2D planes also the forward
     // values of two-pass segments (margins included, at most twice a pass's
     // whole chunks of forward values).  A fused scoring task's columns pass

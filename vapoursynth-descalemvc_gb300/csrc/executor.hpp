@@ -103,9 +103,10 @@ class Executor;
 
 // One launch group of a batch: every job of the group runs in one kernel
 // launch.  `key` identifies the kernel variant (pass, kind, half-bandwidth,
-// input and output sample kinds, window variant); `kind` 0/1 are the
-// sequential Float32/Float64 kernels, 2 the streaming 1D kernels, 3 the
-// transposing streaming 2D kernels.
+// input and output sample kinds, variant); `kind` 0/1 are the sequential
+// Float32/Float64 kernels, 2 the streaming 1D kernels, 3 and 4 the
+// chunk-delayed 2D kernels, 5 and 6 the two-pass Float32/Float64 kernels, 10 the
+// one-axis kernels with the ring in tensor memory.
 struct BatchGroup {
     std::array<int, 6> key{};
     int kind = 0;
@@ -117,8 +118,10 @@ struct BatchGroup {
 };
 
 // CTA sizes chosen per launch-group key (an autotuner's output); groups not
-// listed keep their kernel's default.  Kinds 0/1 accept 32..128, kind 3
-// 32..256 (multiples of 32); kind 2 has a fixed size.
+// listed keep their kernel's default.  Kinds 0/1 accept 32..128, kinds 3 to 6
+// 32..256 (multiples of 32); kinds 2 and 10 have a fixed size and may not be
+// listed.  The launches with the ring in tensor memory (BatchGroup::per_lane)
+// have one CTA size: theirs is accepted and has no effect.
 using BatchTuning = std::map<std::array<int, 6>, int>;
 
 // A batch routed and packed once, with its own job table, scratch and status

@@ -12,8 +12,8 @@ namespace dsmvc_gb {
 
 struct StreamPack {
     bool eligible = false;          // the plan may use the chunk-delayed streaming kernels
-    bool exact = false;             // the plan may use the two-pass transposing kernels
-                                    // (per-destination refill; grouped when ring_ok_transposed)
+    bool exact = false;             // the plan may use the two-pass transposing kernels (on the
+                                    // ring in tensor memory where ring_window is not 0)
     std::string reason;             // why not chunk-delayed, when not
     int window = 0;                 // dense gather window (multiple of 4)
     int forward_stride = 0;         // floats per forward record
@@ -31,8 +31,8 @@ struct StreamPack {
     // its forward substitution from a zero history one chunk early.  Admitted
     // when that warm-up leaves a history influence below 2^-26 per slot
     // (every chunk that can serve as warm-up, computed in double).
-    // Grouped forward records of the chunk-delayed transposing kernels
-    // (tstream_impl.cuh, K = group_union), when the window starts of every
+    // Grouped forward records of the fused scoring kernels (tscore_impl.cuh,
+    // K = group_union), when the window starts of every
     // four consecutive destinations 4g..4g+3 span at most 12 (or 16) samples
     // together with the window: per group, [window start of 4g, its ring
     // offset, end of the union actually needed (the refill target), 0],
@@ -92,8 +92,8 @@ int ring_window(int half_bandwidth, int window, int source_size);
 // below 2^-26 per carry slot (computed in double for every chunk of the
 // plan), which keeps the warm-up error within about one float ULP.
 // Records are built when either family admits the plan; the two-pass
-// transposing kernels (tsolve_impl.cuh) need only the window, monotone
-// window starts and the grouped ring replay.
+// transposing kernels (xring_impl.cuh, tsolve_impl.cuh) need only the window,
+// monotone window starts and the ring replay.
 StreamPack pack_stream_plan(const AxisPlan &plan, int chunk, int ring,
                             bool half_bandwidth_supported, bool half_bandwidth_supported_exact = false);
 

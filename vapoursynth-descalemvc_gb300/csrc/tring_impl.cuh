@@ -171,9 +171,9 @@ struct RingFeeder {
     // word a lane, 128 contiguous bytes a warp-wide copy, where TMA would put it, zeros
     // past the vectors' end.  By cp.async where the vectors begin at a word.  A lane
     // loading its own vector's next 16 samples, unstaged, waited on memory at each
-    // step: one GB300, eight 1919x1079 Float32 planes' rows 219 -> 80 us, sixteen 1079x607
-    // planes 67 -> 53, 24 YUV420P8 frames of 720x480 with tight rows 90 -> 80 (a lone frame
-    // of 8-bit rows that begin inside a word 23 -> 26: its copies wait), and without
+    // step: one GB300, eight 1919x1079 Float32 planes' rows 219 -> 70 us, sixteen 1079x607
+    // planes 67 -> 55, 24 YUV420P8 frames of 720x480 with tight rows 90 -> 81 (a lone frame
+    // of 8-bit rows that begin inside a word 23 -> 25: its copies wait), and without
     // those loads in every refill 64 aligned YUV420P16 1080p frames 536 -> 526.
     static __device__ __noinline__ void copy_words(const StreamJob *job, int first, int next, int size, int count,
                                                    unsigned to, unsigned mb) {
@@ -401,7 +401,8 @@ template <int HB, int W> struct RingRecord {
 // ---- substitutions ---------------------------------------------------------------
 
 // Destinations per iteration of the substitution loops (each iteration moves
-// its histories; one vector a lane spills with more).
+// its histories; one vector a lane spills with more).  Even so half-bandwidth 7 spills
+// at one vector (up to 40 bytes stored and 120 loaded a lane).
 template <int V> constexpr int kRingGroup = V == 2 ? 16 : 8;
 
 template <int N> __device__ __forceinline__ void rload(float (&c)[N], const float *from) {

@@ -20,7 +20,9 @@
 // What bounds them: a half-bandwidth 9 result takes 36 FMA slots (two 16-tap
 // gathers cannot share a packed FMA in this order) and nine 16-byte record
 // loads of two shared-memory cycles each; small launches wait on one vector's
-// chain.  Measured on one GB300 against the kernels with ring in shared memory
+// chain.  Both lane counts spill under their caps of 128 and 168 registers: at
+// half-bandwidths 9 and 11, 40-80 bytes stored and 76-136 loaded a lane at one vector,
+// 100-140 and 216-280 at two, whose loops take 16 destinations at a time.  Measured on one GB300 against the kernels with ring in shared memory
 // and a refill per destination: eight 4K Float32 frames to 1440p, Spline64 blur
 // 1.1, 859 -> 447 us; a 1080p sweep of 189 candidates, of which 33 run these,
 // 3911 -> 3084.
