@@ -78,8 +78,10 @@ struct StreamPack {
     std::vector<int> ring_first_block;   // as chunk_first_block, for these windows
 };
 
-// Longest source that the refill target's field can count.
-constexpr int kRingMaxSource = 1 << 28;
+// Longest source of these records: its blocks, and one more, fit the refill
+// target's 24 bits.
+constexpr int kRingMaxSource = 1 << 27;
+static_assert(kRingMaxSource / 16 + 1 < 1 << 24);
 
 // The compiled window that serves a plan's window in the kernels with the
 // ring in tensor memory; 0 when none does.
