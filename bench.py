@@ -42,11 +42,11 @@ FRAMES = 64
 KERNEL = dict(kernel="lanczos", taps=3, b=0.0, c=0.5, blur=1.0, border="repeat", f64_mode=0)
 METRIC = "descale Mpix/s (source pixels, Delanczos YUV420P16 1920x1080->1440x810)"
 # DRAM bytes (read + write) per frame of both passes: dram__bytes_read.sum +
-# dram__bytes_write.sum of the rows and columns pass from one ncu capture of
-# a 24-frame cut of this workload, divided by 24 (traffic grows with the
-# frame count).
-DRAM_BYTES_PER_FRAME = 619.8e6 / 24
-TRAFFIC_SOURCE = ("ncu capture (dram__bytes_read.sum + dram__bytes_write.sum, both passes) of a "
+# dram__bytes_write.sum of the rows and columns passes of both parts from one ncu
+# capture of a 24-frame cut of this workload (profiles/tring_c1_24frames.md),
+# divided by 24 (traffic grows with the frame count).
+DRAM_BYTES_PER_FRAME = 557.2e6 / 24
+TRAFFIC_SOURCE = ("ncu capture (dram__bytes_read.sum + dram__bytes_write.sum, both passes, both parts) of a "
                   "24-frame cut of this workload, scaled to the step's frames")
 
 
