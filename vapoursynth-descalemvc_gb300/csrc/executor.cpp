@@ -782,8 +782,9 @@ constexpr int kPairingWarps = 8, kPairingRanges = 10;
 // One-axis passes in segments: two chunks of zero-history warm-up, each of which
 // leaves below 2^-26 a slot, leave below half-bandwidth x 2^-52 of a history in each.
 // On every vector tried (test_one_axis, test_gpu_ring.py) a segment's values were
-// then the whole vector's bits; nothing guarantees it.  Ranges of at least three chunks (two cost two 1080p planes 2 us of
-// 25 in repeated work; four cost one plane 2 of 21 in latency).
+// then the whole vector's bits; nothing guarantees it.  Ranges of at least three
+// chunks (two cost two 1080p planes 2 us of 25 in repeated work; four cost one plane
+// 2 of 21 in latency).
 constexpr int kAxisMargin = 2, kAxisMinChunks = 3;
 
 // The kinds with the ring in tensor memory: the 2D passes' 3, whose vectors a
@@ -2332,8 +2333,8 @@ std::size_t PreparedBatch::parts() const { return impl_->parts.size(); }
 
 std::size_t Executor::batch_scratch_bound(const std::vector<PlaneTask> &tasks) {
     // Per task: the intermediate plane (destinations of the first pass x
-    // sources of the second, rows padded to 4, or to tiles of 32) plus a forward plane of the
-    // output's size, in the route's sample width; 2D planes also the forward
+    // sources of the second, rows padded to 4, or to tiles of 32) plus a forward
+    // plane of the output's size, in the route's sample width; 2D planes also the forward
     // values of two-pass segments (margins included, at most twice a pass's
     // whole chunks of forward values).  A fused scoring task's columns pass
     // needs nothing beyond the intermediate.

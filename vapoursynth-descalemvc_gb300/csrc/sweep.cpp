@@ -651,10 +651,10 @@ struct Sweep::Impl {
     }
 
     // Times the first wave's descale with the vectors a lane that each launch's
-    // size gives it and, where that mixes one and two or two may be faster, with
-    // one and with two in all of them, then every launch group of it at each
-    // candidate CTA size, and the scoring column pass at each row
-    // segment (unfused candidates); keeps the fastest of each.  Scores do
+    // size gives it and with one and with two in all of them (where that is
+    // another choice), then every launch group of it at each candidate CTA size,
+    // and the scoring column pass at each row segment (unfused candidates); keeps
+    // the fastest of each.  Scores do
     // not depend on the choices: every kernel variant gives each output bit
     // for bit, and the fused scoring kernel has one launch shape.
     void autotune() {
